@@ -139,7 +139,7 @@ extern "C" int xk_device_info(char *buf, int32_t len)
 // model object
 
 enum { LAYOUT_BITS2D = 1, LAYOUT_BYTES = 2, LAYOUT_CELLS64 = 3, LAYOUT_MASS = 4, LAYOUT_VM = 5, LAYOUT_LCOLOR = 6,
-       LAYOUT_NOISE = 7, LAYOUT_GRAVITY = 8 };
+       LAYOUT_NOISE = 7, LAYOUT_GRAVITY = 8, LAYOUT_BITSND = 9 };
 
 // largest float t with (double)u < p  <=>  u <= t for every float u
 static float below_threshold(double p)
@@ -160,6 +160,7 @@ struct xk_model {
     int layout = 0;
     LifeGeo lg;
     NdGeo ng;
+    BitsNdGeo bg;                // LAYOUT_BITSND (lg: its packing, n / W rows)
     uint32_t *bits[2] = {nullptr, nullptr};
     uint8_t *bytes[2] = {nullptr, nullptr};
     uint64_t *cells64[2] = {nullptr, nullptr};  // EvoLife, GraviCowboys: reference layout, ping-pong
@@ -202,6 +203,12 @@ struct xk_model {
     cudaStream_t copy_stream = nullptr;
     cudaEvent_t rendered[kFrameRing] = {}, copied[kFrameRing] = {};
 };
+
+// bit-packed rows described by m->lg
+static bool bits_layout(const xk_model *m)
+{
+    return m->layout == LAYOUT_BITS2D || m->layout == LAYOUT_BITSND;
+}
 
 static int64_t cells_of(const xk_desc &d)
 {
@@ -571,10 +578,19 @@ extern "C" int xk_model_create(const xk_desc *desc, xk_model **out)
             m->ng.border_state = (uint32_t)border_state;
             for (int i = 0; i < d.ndim; ++i) m->ng.size[i] = d.size[i];
             memcpy(m->ng.delta, d.delta, sizeof(m->ng.delta));
-            const size_t bytes = ((size_t)n + 15) / 16 * 16 + 16;
-            XK_TRY(cudaMalloc(&m->bytes[0], bytes));
-            XK_TRY(cudaMalloc(&m->bytes[1], bytes));
-            XK_TRY(cudaMemsetAsync(m->bytes[0], 0, bytes, m->stream));
+            if (d.family == XK_FAMILY_LIFE && xk_bits_nd_geo(m->ng, &m->bg)) {
+                m->layout = LAYOUT_BITSND;
+                m->lg = xk_life_geo(d.size[0], n / d.size[0], d.torus, border_state);
+                const size_t words = (size_t)m->bg.words;
+                XK_TRY(cudaMalloc(&m->bits[0], (words + 4) * 4));
+                XK_TRY(cudaMalloc(&m->bits[1], (words + 4) * 4));
+                XK_TRY(cudaMemsetAsync(m->bits[0], 0, (words + 4) * 4, m->stream));
+            } else {
+                const size_t bytes = ((size_t)n + 15) / 16 * 16 + 16;
+                XK_TRY(cudaMalloc(&m->bytes[0], bytes));
+                XK_TRY(cudaMalloc(&m->bytes[1], bytes));
+                XK_TRY(cudaMemsetAsync(m->bytes[0], 0, bytes, m->stream));
+            }
         }
         if (m->layout != LAYOUT_CELLS64 && m->layout != LAYOUT_MASS && m->layout != LAYOUT_VM &&
             m->layout != LAYOUT_LCOLOR && m->layout != LAYOUT_NOISE && m->layout != LAYOUT_GRAVITY)
@@ -645,7 +661,7 @@ extern "C" int xk_upload(xk_model *m, const void *host_main, int64_t ncells)
     XK_CUDA(cudaMemcpyAsync(m->stage, host_main, (size_t)m->n * esz, cudaMemcpyHostToDevice,
                             m->stream));
     unsigned int *bad;
-    if (m->layout == LAYOUT_BITS2D) {
+    if (bits_layout(m)) {
         XK_CUDA(xk_life_pack(m->stage, esz, m->bits[m->cur], m->lg, m->stream));
         bad = (unsigned int *)(m->bits[m->cur] + (int64_t)m->lg.H * m->lg.wpr);
     } else {
@@ -685,7 +701,7 @@ extern "C" int xk_download(xk_model *m, void *host_main, int64_t ncells)
         XK_CUDA(cudaStreamSynchronize(m->stream));
         return XK_OK;
     }
-    if (m->layout == LAYOUT_BITS2D)
+    if (bits_layout(m))
         XK_CUDA(xk_life_unpack(m->bits[m->cur], m->stage, esz, m->lg, m->stream));
     else
         XK_CUDA(xk_nd_unpack(m->bytes[m->cur], m->stage, esz, m->n, m->stream));
@@ -714,7 +730,7 @@ static int materialize_colors(xk_model *m)
     }
     if (!m->derived) return XK_OK;
     const int smooth = m->d.color_kind == XK_COLOR_MOVING_AVERAGE ? m->d.smooth : 1;
-    if (m->layout == LAYOUT_BITS2D)
+    if (bits_layout(m))
         XK_CUDA(xk_life_colors(m->bits[m->cur], m->col, m->lg, m->lut, smooth, m->stream));
     else
         XK_CUDA(xk_nd_colors(m->bytes[m->cur], m->col, m->n, m->lut, smooth, m->stream));
@@ -797,7 +813,7 @@ static int life_color_step(xk_model *m)
 {
     if (m->d.color_kind == XK_COLOR_NONE) return XK_OK;
     const int plain = m->d.color_kind == XK_COLOR_PLAIN;
-    if (m->layout == LAYOUT_BITS2D)
+    if (bits_layout(m))
         XK_CUDA(xk_life_color_step(m->bits[m->cur], m->col, m->lg, m->lut, m->d.fade_in,
                                    m->d.fade_out, m->d.smooth, plain, m->stream));
     else
@@ -959,7 +975,10 @@ static int step_enqueue(xk_model *m, int64_t first, int64_t count, uint8_t *fram
                     m->cur = 1 - m->cur;
                 }
             } else {
-                if (m->d.family == XK_FAMILY_SHIFT)
+                if (m->layout == LAYOUT_BITSND)
+                    XK_CUDA(xk_life_step_bits_nd(m->bits[m->cur], m->bits[1 - m->cur], m->bg, m->rule0,
+                                                 m->rule1, m->stream));
+                else if (m->d.family == XK_FAMILY_SHIFT)
                     XK_CUDA(xk_shift_step_nd(m->bytes[m->cur], m->bytes[1 - m->cur], m->ng, (int)m->rule0,
                                              m->stream));
                 else

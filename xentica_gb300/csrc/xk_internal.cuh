@@ -210,6 +210,28 @@ struct NdGeo {
     int8_t delta[XK_MAXNBR][XK_MAXDIM];
     uint32_t border_state;      // 0/1 state of off-board cells
 };
+// bit-packed along axis 0 (life_nd.cu): n / W rows of wpr words, neighbours
+// grouped by row (delta[k][1..]; delta[k][0]: bit 0 the left, 1 the middle, 2
+// the right cell of the row)
+struct BitsNdGeo {
+    int32_t ndim, nbr, groups, torus, moore3d;
+    int32_t size[XK_MAXDIM];
+    int8_t delta[XK_MAXNBR][XK_MAXDIM];
+    int32_t wpr, rlast;
+    uint32_t lastmask, bfill;
+    uint32_t words;             // rows * wpr
+    uint32_t div_wpr, div_h;    // xk_div_magic(wpr, words); 3-D: xk_div_magic(size[1], rows)
+};
+// the rule over the neighbour count 0..31 as LifeTable's coefficients: pair
+// q < 16 (dead 2q, 2q + 1), q >= 16 the same for live cells
+struct LifeTable32 {
+    uint32_t a[32], k[32];
+};
+// the bit-packed form of a lattice; 0 where its kernels do not apply (offsets
+// of more than one cell, more than 2^31 words)
+int xk_bits_nd_geo(const NdGeo &nd, BitsNdGeo *out);
+cudaError_t xk_life_step_bits_nd(const uint32_t *src, uint32_t *dst, const BitsNdGeo &g, uint32_t rule0,
+                                 uint32_t rule1, cudaStream_t s);
 cudaError_t xk_nd_pack(const void *src, int esz, uint8_t *dst, int64_t n, cudaStream_t s);
 cudaError_t xk_nd_unpack(const uint8_t *src, void *dst, int esz, int64_t n, cudaStream_t s);
 cudaError_t xk_life_step_nd(const uint8_t *src, uint8_t *dst, const NdGeo &g, uint32_t rule0,
