@@ -77,3 +77,33 @@ def test_frames_vs_oracle_render():
         O.noise_run(topo, fld, col, 1, color=O._color(True, 40, 25, 1))
         img = O.render(topo, col, size[0], size[1], smooth=1).astype(np.uint8)
         assert np.array_equal(frames[g], img), g
+
+
+@pytest.mark.parametrize("size", [(128, 1), (127, 1), (43, 3), (33, 31), (1, 1), (257, 5)])
+@pytest.mark.parametrize("shift", [0, 1, 3])
+def test_device_frames_at_any_alignment(size, shift):
+    """Many frames from one launch, whole and partial warps, frames that start
+    at every offset from a word, grey cells and coloured ones."""
+    torch = pytest.importorskip("torch")
+    model = NoiseTV(type("E", (NoiseExperiment, ), {"size": size}))
+    n = model.cells_num
+    rng = np.random.RandomState(n + shift)
+    cells = rng.randint(0, 65535, n).astype(np.uint16)
+    colors = np.repeat(rng.randint(0, 256, n), 3).astype(np.int32)
+    colors[:3 * (n // 3)] += rng.randint(0, 2, 3 * (n // 3)).astype(np.int32) * (shift != 1)
+    model.gpu.load(cells, colors)
+    model.set_viewport(size)
+    out = torch.full((5 * 3 * n + 16, ), 77, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()        # the fill runs on another stream than the model
+    model.gpu.step_frames(5, size[0], size[1], 1, 0, 0, out.data_ptr() + 4 + shift, on_device=True)
+    got = out.cpu().numpy()
+    assert (got[:4 + shift] == 77).all() and (got[4 + shift + 15 * n:] == 77).all()
+    topo = O.Topology(size)
+    fld, col = topo.field(cells, np.uint16), colors.copy()
+    for g in range(5):
+        O.noise_run(topo, fld, col, 1, color=O._color(True, 40, 25, 1))
+        img = O.render(topo, col, size[0], size[1], smooth=1).astype(np.uint8)
+        at = 4 + shift + 3 * n * g
+        assert np.array_equal(got[at:at + 3 * n], img.ravel()), g
+    assert np.array_equal(model.gpu.arrays.cells.get()[:n], fld[:n])
+    assert np.array_equal(model.gpu.arrays.colors.get(), col)

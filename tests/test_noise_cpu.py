@@ -34,3 +34,18 @@ def test_template_choice():
         assert d.ndim == ndim and d.state_bytes == 2
         assert (d.fade_in, d.fade_out, d.smooth) == (40, 25, 1)
         assert d.color_kind == nat.XK_COLOR_MOVING_AVERAGE
+
+
+def test_grey_level_and_advance_in_integers():
+    """The kernel's integer forms (csrc/noise.cu) equal the reference's float
+    grey level for every state and its two advances for every 16-bit state."""
+    x = np.arange(65535)
+    want = (x.astype(np.float32) / np.float32(65535) * np.float32(255)).astype(np.uint32)
+    assert np.array_equal((x * 65281) % 2 ** 32 >> 24, want)
+    x = np.arange(65536)
+    one = (x * 58321 + 11113) % 65535
+    two = (one * 58321 + 11113) % 65535
+    t = (58321 ** 2 % 65535) * x + (58321 * 11113 + 11113) % 65535
+    assert t.max() < 2 ** 32
+    s = (t & 65535) + (t >> 16)
+    assert np.array_equal(np.where(s >= 65535, s - 65535, s), two)

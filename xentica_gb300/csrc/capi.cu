@@ -867,10 +867,11 @@ static bool shift_jump_enabled()
     return !(v && v[0] == '0');
 }
 
-// frame (EvoLife, count == 1 only): the generation's zoom-1 frame written by
-// the step kernel itself; proj (mass transfer, count == 1 only): the step
-// kernel also adds the new state's column colour sums into it, and with
-// frame_prev writes the previous generation's frame from proj_prev
+// frame (fused families): the zoom-1 frame of every generation written by the
+// step kernel itself, one after another (count == 1 but for noise); proj
+// (mass transfer, count == 1 only): the step kernel also adds the new state's
+// column colour sums into it, and with frame_prev writes the previous
+// generation's frame from proj_prev
 static int step_enqueue(xk_model *m, int64_t first, int64_t count, uint8_t *frame = nullptr,
                         uint32_t *proj = nullptr, uint32_t *proj_prev = nullptr, uint8_t *frame_prev = nullptr)
 {
@@ -898,10 +899,12 @@ static int step_enqueue(xk_model *m, int64_t first, int64_t count, uint8_t *fram
         return XK_OK;
     }
     if (m->layout == LAYOUT_NOISE) {
-        // cells are independent: up to 1024 generations per launch (one with a frame)
+        // cells are independent: up to 1024 generations per launch, their
+        // frames one after another
         for (int64_t g = 0; g < count;) {
-            const int gens = frame ? 1 : (int)std::min<int64_t>(1024, count - g);
-            XK_CUDA(xk_noise_step(m->cells16, m->col, m->d, m->n, gens, m->stream, frame, m->d.render_smooth));
+            const int gens = (int)std::min<int64_t>(1024, count - g);
+            XK_CUDA(xk_noise_step(m->cells16, m->col, m->d, m->n, gens, m->stream,
+                                  frame ? frame + 3 * m->n * g : nullptr, m->d.render_smooth));
             g += gens;
         }
         return XK_OK;
@@ -1273,7 +1276,13 @@ extern "C" int xk_step_frames(xk_model *m, int64_t nsteps, int32_t width, int32_
         rc = mass_frames_enqueue(m, nsteps, frames, frames_on_device != 0, fb);
         if (rc != XK_OK) return rc;
     }
-    for (int64_t g = 0; g < nsteps && !mass_fused; ++g) {
+    // device frames of noise: one launch writes many
+    const bool whole_call = fused && frames_on_device && m->layout == LAYOUT_NOISE;
+    if (whole_call) {
+        rc = step_enqueue(m, 0, nsteps, frames);
+        if (rc != XK_OK) return rc;
+    }
+    for (int64_t g = 0; g < nsteps && !mass_fused && !whole_call; ++g) {
         const int k = (int)(g % kFrameRing);
         uint8_t *dst = frames_on_device ? frames + (size_t)g * fb : m->ring + (size_t)k * fb;
         if (!frames_on_device && g >= kFrameRing)

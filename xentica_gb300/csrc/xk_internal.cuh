@@ -294,9 +294,10 @@ cudaError_t xk_lifecolor_step(const uint32_t *src, uint32_t *dst, int32_t *col, 
                               cudaStream_t s, uint8_t *frame = nullptr, int frame_smooth = 0);
 
 // per-cell noise (noise.cu): `generations` generations of every cell in one
-// launch, in place (1 when the zoom-1 frame of a 2-D lattice is written)
+// launch, in place; frames: null, or the zoom-1 frames of a 2-D lattice, one
+// per generation, 3 n bytes each
 cudaError_t xk_noise_step(uint16_t *cells, int32_t *col, const xk_desc &d, int64_t n, int generations,
-                          cudaStream_t s, uint8_t *frame = nullptr, int frame_smooth = 0);
+                          cudaStream_t s, uint8_t *frames = nullptr, int frame_smooth = 0);
 // one GraviCowboys generation, cells ping-pong (gravity.cu)
 cudaError_t xk_gravity_step(const uint64_t *src, uint64_t *dst, int32_t *col, const xk_desc &d,
                             cudaStream_t s, uint8_t *frame, int frame_smooth);
