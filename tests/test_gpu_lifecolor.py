@@ -87,3 +87,28 @@ def test_frames_vs_oracle_render():
         O.lifecolor_run(topo, fld, col, 1, color=O._color(True, 255, 10, 1))
         img = O.render(topo, col, size[0], size[1], smooth=1).astype(np.uint8)
         assert np.array_equal(frames[g], img), g
+
+
+@pytest.mark.parametrize("size", [(1, 1), (3, 25), (121, 24), (119, 26), (124, 9), (250, 57), (480, 640), (363, 601)])
+@pytest.mark.parametrize("cls,border", [(GameOfLifeColor, None), (GameOfLifeColorStatic, STATIC)])
+def test_several_generations_a_launch(cls, border, size):
+    """Tile edges (120 columns, 8 or 24 rows inside), rows that do not start on
+    a word, device frames from launches of 4, 4 and 3 generations, colours in
+    and out of the range where a pixel is the colour's low byte."""
+    torch = pytest.importorskip("torch")
+    model, cells, colors = _random_model(cls, size, size[0] + 7 * size[1])
+    n = model.cells_num
+    colors[::7] += np.int32(1 << 24)
+    model.gpu.load(cells, colors)
+    model.set_viewport(size)
+    out = torch.empty((11, 3 * n), dtype=torch.uint8, device="cuda")
+    model.gpu.step_frames(11, size[0], size[1], 1, 0, 0, out.data_ptr(), on_device=True)
+    frames = out.cpu().numpy()
+    topo = O.Topology(size, "moore", border)
+    fld, col = topo.field(cells, np.uint32), colors.copy()
+    for g in range(11):
+        O.lifecolor_run(topo, fld, col, 1, color=O._color(True, 255, 10, 1))
+        img = O.render(topo, col, size[0], size[1], smooth=1).astype(np.uint8)
+        assert np.array_equal(frames[g], img.ravel()), g
+    assert np.array_equal(model.gpu.arrays.cells.get()[:n], fld[:n])
+    assert np.array_equal(model.gpu.arrays.colors.get(), col)

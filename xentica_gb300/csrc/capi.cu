@@ -868,7 +868,8 @@ static bool shift_jump_enabled()
 }
 
 // frame (fused families): the zoom-1 frame of every generation written by the
-// step kernel itself, one after another (count == 1 but for noise); proj
+// step kernel itself, one after another (count == 1 for EvoLife and
+// GraviCowboys); proj
 // (mass transfer, count == 1 only): the step kernel also adds the new state's
 // column colour sums into it, and with frame_prev writes the previous
 // generation's frame from proj_prev
@@ -918,10 +919,13 @@ static int step_enqueue(xk_model *m, int64_t first, int64_t count, uint8_t *fram
         return XK_OK;
     }
     if (m->layout == LAYOUT_LCOLOR) {
-        for (int64_t g = 0; g < count; ++g) {
-            XK_CUDA(xk_lifecolor_step(m->cells32[m->cur], m->cells32[1 - m->cur], m->col, m->d, m->stream,
-                                      frame, m->d.render_smooth));
+        for (int64_t g = 0; g < count;) {
+            const int gens = (int)std::min<int64_t>(xk_lifecolor_max_generations(), count - g);
+            XK_CUDA(xk_lifecolor_step(m->cells32[m->cur], m->cells32[1 - m->cur], m->col, m->d, gens, m->col_range,
+                                      m->stream, frame ? frame + 3 * m->n * g : nullptr,
+                                      m->d.render_smooth));
             m->cur = 1 - m->cur;
+            g += gens;
         }
         return XK_OK;
     }
@@ -1276,8 +1280,8 @@ extern "C" int xk_step_frames(xk_model *m, int64_t nsteps, int32_t width, int32_
         rc = mass_frames_enqueue(m, nsteps, frames, frames_on_device != 0, fb);
         if (rc != XK_OK) return rc;
     }
-    // device frames of noise: one launch writes many
-    const bool whole_call = fused && frames_on_device && m->layout == LAYOUT_NOISE;
+    // device frames of noise and colour Life: one launch writes several
+    const bool whole_call = fused && frames_on_device && (m->layout == LAYOUT_NOISE || m->layout == LAYOUT_LCOLOR);
     if (whole_call) {
         rc = step_enqueue(m, 0, nsteps, frames);
         if (rc != XK_OK) return rc;

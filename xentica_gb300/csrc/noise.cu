@@ -20,11 +20,12 @@
 //
 // Bound by instruction issue without frames, by the frames' writes with them.
 // 1920 x 1080, a frame every generation: one launch a generation took 9.8 us
-// (state, colours and frame through L2, 26.8 warp instructions a cell), now 2.2.
+// (state, colours and frame through L2, 26.8 warp instructions a cell), now 1.8.
 // (Measured and not kept: the grey level of every x from a 65 535-byte table,
 // which put a load in each generation's dependent chain.)
-#include "frame.cuh"
 #include "xk_internal.cuh"
+
+#include "frame.cuh"
 
 struct NoiseParams {
     int64_t n;
@@ -33,6 +34,7 @@ struct NoiseParams {
     int32_t generations;         // generations per launch
     uint8_t *frames;             // the zoom-1 RendererPlain frames of a 2-D lattice, 3 n bytes each
     int32_t frame_smooth;        // their SMOOTH_FACTOR (0: none)
+    int32_t small;               // xk_px_stays_small
 };
 
 // the two advances of a generation composed: 58321^2 and 58321 * 11113 + 11113, mod 65535
@@ -49,8 +51,8 @@ __device__ __forceinline__ uint32_t xk_noise_advance(uint32_t x)
 __device__ __forceinline__ int xk_noise_grey(uint32_t x) { return (int)((x * 65281u) >> 24); }
 
 // the generations of a thread's four cells; CH: colour channels computed (1:
-// all equal)
-template <bool FRAME, int CH>
+// all equal); SMALL: a pixel is its colour's low byte
+template <bool FRAME, int CH, bool SMALL>
 __device__ __forceinline__ void xk_noise_cells(uint32_t x[4], int c[4][3], const NoiseParams &p, int64_t i,
                                                int lane, bool whole_warp)
 {
@@ -68,10 +70,11 @@ __device__ __forceinline__ void xk_noise_cells(uint32_t x[4], int c[4][3], const
 #pragma unroll
             for (int k = 0; k < 4; ++k)
 #pragma unroll
-                for (int ch = 0; ch < 3; ++ch) r[ch][k] = ch < CH ? xk_pixel(c[k][ch], p.frame_smooth) : r[0][k];
+                for (int ch = 0; ch < 3; ++ch)
+                    r[ch][k] = ch >= CH ? r[0][k] : SMALL ? (uint32_t)c[k][ch] : xk_pixel(c[k][ch], p.frame_smooth);
             if (whole_warp) {
                 xk_pack_px4(r[0], r[1], r[2], w);
-                xk_store_px4(px, w, lane);
+                xk_store_px4(px, w, lane, 0, 31);
             } else {
 #pragma unroll
                 for (int k = 0; k < 4; ++k)
@@ -122,13 +125,24 @@ xk_k_noise(uint16_t *__restrict__ cells, int32_t *__restrict__ col, NoiseParams 
             }
     }
     if (ma) {
-        bool grey = true;
+        bool grey = true, small = p.small != 0;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) grey = grey && c[k][0] == c[k][1] && c[k][0] == c[k][2];
+        for (int k = 0; k < 4; ++k) {
+            grey = grey && c[k][0] == c[k][1] && c[k][0] == c[k][2];
+            small = small && xk_px_small(c[k][0]) && xk_px_small(c[k][1]) && xk_px_small(c[k][2]);
+        }
         // one form for a whole warp: its frame stores are the warp's
-        if (whole_warp) grey = __all_sync(0xFFFFFFFFu, grey);
-        if (grey) xk_noise_cells<FRAME, 1>(x, c, p, i, lane, whole_warp);
-        else xk_noise_cells<FRAME, 3>(x, c, p, i, lane, whole_warp);
+        if (whole_warp) {
+            grey = __all_sync(0xFFFFFFFFu, grey);
+            small = __all_sync(0xFFFFFFFFu, small);
+        }
+        if (!FRAME || !small) {
+            if (!FRAME && grey) xk_noise_cells<FRAME, 1, false>(x, c, p, i, lane, whole_warp);
+            else xk_noise_cells<FRAME, 3, false>(x, c, p, i, lane, whole_warp);
+        } else {
+            if (grey) xk_noise_cells<FRAME, 1, true>(x, c, p, i, lane, whole_warp);
+            else xk_noise_cells<FRAME, 3, true>(x, c, p, i, lane, whole_warp);
+        }
     } else {
         for (int g = 0; g < p.generations; ++g)
 #pragma unroll
@@ -167,6 +181,7 @@ cudaError_t xk_noise_step(uint16_t *cells, int32_t *col, const xk_desc &d, int64
     p.generations = generations;
     p.frames = frames;
     p.frame_smooth = frame_smooth;
+    p.small = xk_px_stays_small(d, frame_smooth);
     const int threads = 256;
     const dim3 grid((unsigned)((n + 4 * threads - 1) / (4 * threads)));
     return frames ? xk_launch_pdl(xk_k_noise<true>, grid, dim3(threads), 0, s, cells, col, p)

@@ -288,10 +288,13 @@ cudaError_t xk_evolife_step(const uint64_t *src, uint64_t *dst, int32_t *col, co
                             float mut_thresh, cudaStream_t s, uint8_t *frame = nullptr,
                             int frame_smooth = 0);
 
-// Life with inherited colour channels (lifecolor.cu): one generation, the
-// colours updated, and (frame) the zoom-1 frame as for EvoLife
-cudaError_t xk_lifecolor_step(const uint32_t *src, uint32_t *dst, int32_t *col, const xk_desc &d,
-                              cudaStream_t s, uint8_t *frame = nullptr, int frame_smooth = 0);
+// Life with inherited colour channels (lifecolor.cu): 1 .. max generations,
+// src -> dst, the colours updated, and (frames) each one's zoom-1 frame, one
+// after another; color_range: smallest and largest colour that was loaded
+int xk_lifecolor_max_generations();
+cudaError_t xk_lifecolor_step(const uint32_t *src, uint32_t *dst, int32_t *col, const xk_desc &d, int generations,
+                              const int32_t color_range[2], cudaStream_t s, uint8_t *frames = nullptr,
+                              int frame_smooth = 0);
 
 // per-cell noise (noise.cu): `generations` generations of every cell in one
 // launch, in place; frames: null, or the zoom-1 frames of a 2-D lattice, one
