@@ -1,0 +1,173 @@
+"""The interpreter's 32-bit form against its general one: random programs of
+every operation and 32-bit type, on edge values, run in both forms (one
+instruction of a 64-bit type keeps a program on the general form)."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from xentica_gb300 import _native as nat
+from xentica_gb300.core import ir, vm
+
+pytestmark = pytest.mark.gpu
+
+BOOL, U8, U16, I32, U32, I64, F32 = 0, 1, 2, 3, 4, 5, 7
+O = vm.OP
+EDGE = [0, 1, 2, 3, 7, 31, 32, 33, 127, 255, 256, 65535, 65536, 2 ** 31 - 1, 2 ** 31, 2 ** 31 + 1,
+        2 ** 32 - 1, 2 ** 32 - 2]
+FLOATS = [0.0, -0.0, 0.5, -0.5, 1.0, -1.0, 255.9, 65536.5, -3.7, 2.5e9, 5e9, -5e9, 1e20, -1e20,
+          float("inf"), float("-inf"), float("nan")]
+
+
+class _Random:
+    """A straight-line program whose operands have the types its operations
+    name, as the compiler's do, registers reused at random."""
+
+    def __init__(self, seed, nbr, esz, absorb, nregs=24):
+        self.r = np.random.RandomState(seed)
+        self.nbr, self.esz, self.absorb, self.nregs = nbr, esz, absorb, nregs
+        self.code, self.consts, self.types = [], [], {}
+
+    def emit(self, op, ty, a=0, b=0, c=0, result=None):
+        dst = int(self.r.randint(self.nregs))
+        self.code.append((O[op], ty, dst, a, b, c, 0))
+        self.types[dst] = ty if result is None else result
+
+    def pick(self, types):
+        regs = [q for q, t in self.types.items() if t in types]
+        return int(regs[self.r.randint(len(regs))]) if regs else None
+
+    def load(self):
+        kind = int(self.r.randint(4))
+        k = int(self.r.randint(self.nbr)) if kind >= 2 else 0
+        ty = {1: U8, 2: U16, 4: U32}[self.esz]
+        # what the pass does not write in other cells: emit the main plane,
+        # absorb the neighbours' buffers and its own planes
+        plane = 0 if not self.absorb else int(self.r.randint(1, self.nbr + 1)) if kind >= 2 else \
+            int(self.r.randint(self.nbr + 1))
+        self.emit("load", ty, kind, k, plane)
+
+    def const(self):
+        ty = int(self.r.choice([I32, U32, F32, U8]))
+        if ty == F32:
+            v = np.float32(FLOATS[self.r.randint(len(FLOATS))])
+        elif ty == U8:
+            v = int(self.r.randint(256))
+        else:
+            v = EDGE[self.r.randint(len(EDGE))]
+            v = v - 2 ** 32 if ty == I32 and v >= 2 ** 31 else v
+        ctype = {I32: ir.I32, U32: ir.U32, F32: ir.F32, U8: ir.U32}[ty]
+        self.consts.append(vm.pack_value(v, ctype))
+        self.emit("const", ty, len(self.consts) - 1)
+
+    def step(self):
+        kind = self.r.randint(12)
+        ints = (BOOL, U8, U16, I32, U32)
+        if kind == 0:
+            return self.const()
+        if kind == 1:
+            a = self.pick(ints + (F32, ))
+            to = int(self.r.choice([BOOL, U8, U16, I32, U32, F32]))
+            return self.emit("cvt", to, a, self.types[a])
+        if kind == 2:
+            a, t = self.pick(ints), int(self.r.choice([I32, U32, F32, U8]))
+            b = self.pick((t, ))
+            c = self.pick((t, ))
+            return self.emit("sel", t, a, b, c) if b is not None else None
+        if kind == 3:
+            a = self.pick((I32, U32, F32))
+            t = self.types[a] if a is not None else None
+            op = str(self.r.choice(["neg", "abs"] if t == F32 else ["neg", "~", "abs"]))
+            return self.emit(op, t, a) if a is not None else None
+        if kind == 4:
+            a = self.pick((U32, ))
+            return self.emit("popc", I32, a) if a is not None else None
+        if kind == 5:
+            a = self.pick((I32, U32, F32, U8, U16))
+            return self.emit("mov", self.types[a], a)
+        t = int(self.r.choice([I32, U32, F32]))
+        a, b = self.pick((t, )), self.pick((t, ))
+        if a is None:
+            return None
+        if t == F32:
+            op = str(self.r.choice(["+", "-", "*", "/", "<", "<=", ">", ">=", "==", "!="]))
+        else:
+            op = str(self.r.choice(["+", "-", "*", "/", "%", "&", "|", "^", "<<", ">>", "<", "<=", ">", ">=",
+                                    "==", "!="]))
+            if op in ("<<", ">>"):
+                b = self.pick((I32, ))
+                if b is None:
+                    return None
+        cmp_op = O["<"] <= O[op] <= O["!="]
+        return self.emit(op, t, a, b, result=I32 if cmp_op else None)
+
+    def program(self, steps, stores, color):
+        for _ in range(3):
+            self.load()
+            self.const()
+        for _ in range(steps):
+            self.step()
+            if self.r.randint(9) == 0:
+                self.load()
+        for plane in stores:
+            a = self.pick((BOOL, U8, U16, I32, U32, F32))
+            self.code.append((O["store"], U32, 0, a, plane, 0, 0))
+            self.step()
+        if color:
+            a, b, c = (self.pick((I32, U32, U8, U16, BOOL)) for _ in range(3))
+            self.code.append((O["color"], I32, 0, a, b, c, 0))
+
+
+def _run(desc, programs, init, col, wide):
+    lib = nat.load()
+    h = ctypes.c_void_p()
+    nat.check(lib.xk_model_create(ctypes.byref(desc), ctypes.byref(h)), "xk_model_create")
+    try:
+        n = init.size
+        for which, p in enumerate(programs):
+            code, consts = list(p.code), list(p.consts)
+            if wide:
+                code.insert(0, (O["const"], I64, p.nregs, 0, 0, 0, 0))
+            code = np.array(code, dtype=vm.INS_DTYPE)
+            consts = np.array(consts, dtype=np.uint64)
+            nat.check(lib.xk_vm_load(h, which, nat.ptr(code), len(code), nat.ptr(consts), len(consts),
+                                     p.nregs + 1), "xk_vm_load")
+        nat.check(lib.xk_upload(h, nat.ptr(init), n), "xk_upload")
+        nat.check(lib.xk_upload_colors(h, nat.ptr(col), n), "xk_upload_colors")
+        nat.check(lib.xk_step(h, 3), "xk_step")
+        cells, out = np.empty_like(init), np.empty_like(col)
+        nat.check(lib.xk_download(h, nat.ptr(cells), n), "xk_download")
+        nat.check(lib.xk_download_colors(h, nat.ptr(out), n), "xk_download_colors")
+    finally:
+        lib.xk_model_destroy(h)
+    return cells, out
+
+
+@pytest.mark.parametrize("seed", range(48))
+def test_random_programs(seed):
+    r = np.random.RandomState(1000 + seed)
+    ndim = int(r.randint(1, 4))
+    size = [int(v) for v in r.choice([1, 2, 3, 5, 8, 33, 64], ndim)]
+    if seed % 6 == 0:
+        size = [257, 41][:ndim] + [2] * (ndim - 2)
+    esz = int(r.choice([1, 2, 4]))
+    desc = nat.XkDesc()
+    desc.abi_version, desc.family, desc.ndim, desc.nbr = nat.XK_ABI_VERSION, nat.XK_FAMILY_VM, ndim, 2 * ndim
+    for d, s in enumerate(size):
+        desc.size[d] = s
+        desc.delta[2 * d][d], desc.delta[2 * d + 1][d] = 1, -1
+    desc.torus, desc.state_bytes = int(seed % 2), esz
+    desc.border_value = int(r.randint(0, 2 ** min(8 * esz, 31)))
+    desc.color_kind = nat.XK_COLOR_MOVING_AVERAGE if seed % 3 else nat.XK_COLOR_PLAIN
+    desc.fade_in, desc.fade_out, desc.smooth = 40, 25, 2
+    n = int(np.prod(size))
+    init = r.choice(np.array(EDGE + [5, 6], dtype=np.uint64), n).astype({1: np.uint8, 2: np.uint16, 4: np.uint32}[esz])
+    col = r.randint(-500, 500, 3 * n).astype(np.int32)
+    emit = _Random(seed, 2 * ndim, esz, False)
+    emit.program(40, range(1, 2 * ndim + 1), False)
+    absorb = _Random(7000 + seed, 2 * ndim, esz, True)
+    absorb.program(120, [0], True)
+    want = _run(desc, (emit, absorb), init, col, True)
+    got = _run(desc, (emit, absorb), init, col, False)
+    assert np.array_equal(got[0], want[0])
+    assert np.array_equal(got[1], want[1])

@@ -192,6 +192,11 @@ struct xk_model {
     xk_vm_ins *vm_code[2] = {nullptr, nullptr};     // emit, absorb
     uint64_t *vm_consts[2] = {nullptr, nullptr};
     int vm_ncode[2] = {0, 0};
+    XkVmNarrow vm_narrow[2];                        // their 32-bit forms, where vm_is_narrow
+    bool vm_is_narrow[2] = {false, false};
+    bool vm_params_fit = true;                      // the bound parameters fit those
+    uint32_t *vm_ncodes[2] = {nullptr, nullptr}, *vm_nconsts[2] = {nullptr, nullptr};
+    uint64_t vm_bound[XK_VM_MAX_PARAMS] = {};
     uint64_t *vm_params = nullptr;                  // XK_VM_MAX_PARAMS slots
     VmGeo vg;
     int hf = 0;                  // colour is a function of the state alone
@@ -402,6 +407,8 @@ static void free_model(xk_model *m)
     for (int i = 0; i < 2; ++i) {
         if (m->vm_code[i]) cudaFree(m->vm_code[i]);
         if (m->vm_consts[i]) cudaFree(m->vm_consts[i]);
+        if (m->vm_ncodes[i]) cudaFree(m->vm_ncodes[i]);
+        if (m->vm_nconsts[i]) cudaFree(m->vm_nconsts[i]);
     }
     if (m->fld) cudaFree(m->fld);
     if (m->vm_params) cudaFree(m->vm_params);
@@ -868,8 +875,8 @@ static bool shift_jump_enabled()
 }
 
 // frame (fused families): the zoom-1 frame of every generation written by the
-// step kernel itself, one after another (count == 1 for EvoLife and
-// GraviCowboys); proj
+// step kernel itself, one after another (count == 1 for EvoLife, GraviCowboys
+// and the interpreter); proj
 // (mass transfer, count == 1 only): the step kernel also adds the new state's
 // column colour sums into it, and with frame_prev writes the previous
 // generation's frame from proj_prev
@@ -878,9 +885,15 @@ static int step_enqueue(xk_model *m, int64_t first, int64_t count, uint8_t *fram
 {
     if (m->layout == LAYOUT_VM) {
         for (int64_t g = 0; g < count; ++g)
-            for (int w = 0; w < 2; ++w)
-                XK_CUDA(xk_vm_run(m->vm_code[w], m->vm_ncode[w], m->vm_consts[w], m->vm_params,
-                                  m->fld, m->col, m->vg, m->stream));
+            for (int w = 0; w < 2; ++w) {
+                if (m->vm_is_narrow[w] && m->vm_params_fit)
+                    XK_CUDA(xk_vm_run_narrow(m->vm_narrow[w], m->vm_ncodes[w], m->vm_nconsts[w], m->vm_params, m->fld,
+                                             m->col, m->vg, m->stream, w == 1 ? frame : nullptr,
+                                             m->d.render_smooth));
+                else
+                    XK_CUDA(xk_vm_run(m->vm_code[w], m->vm_ncode[w], m->vm_consts[w], m->vm_params, m->fld, m->col,
+                                      m->vg, m->stream));
+            }
         return XK_OK;
     }
     if (m->layout == LAYOUT_MASS) {
@@ -1265,8 +1278,11 @@ extern "C" int xk_step_frames(xk_model *m, int64_t nsteps, int32_t width, int32_
         }
     }
     // EvoLife or colour Life viewed whole at zoom 1: the step kernel writes the frame
+    // (on the interpreter the absorb pass, where it has a 32-bit form that colours)
+    const bool vm_frames = m->layout == LAYOUT_VM && m->vm_is_narrow[1] && m->vm_params_fit &&
+                           m->vm_narrow[1].colors;
     const bool fused = (m->layout == LAYOUT_CELLS64 || m->layout == LAYOUT_LCOLOR || m->layout == LAYOUT_NOISE ||
-                        m->layout == LAYOUT_GRAVITY) &&
+                        m->layout == LAYOUT_GRAVITY || vm_frames) &&
                        m->d.color_kind != XK_COLOR_NONE &&
                        m->d.ndim == 2 && m->d.proj_axis0 == 0 && m->d.proj_axis1 == 1 && zoom == 1 &&
                        dx == 0 && dy == 0 && width == m->d.size[0] && height == m->d.size[1];
@@ -1418,6 +1434,20 @@ static bool vm_check(const xk_model *m, const xk_vm_ins &in, int nconsts, int nr
     }
 }
 
+// whether every bound parameter that a 32-bit program reads is the sign or
+// zero extension of its low half
+static bool vm_params_fit(const xk_model *m)
+{
+    for (int w = 0; w < 2; ++w) {
+        if (!m->vm_is_narrow[w]) continue;
+        for (const XkVmParamUse &u : m->vm_narrow[w].params) {
+            const uint64_t v = m->vm_bound[u.slot];
+            if (u.sign ? v != (uint64_t)(int64_t)(int32_t)(uint32_t)v : v >> 32 != 0) return false;
+        }
+    }
+    return true;
+}
+
 extern "C" int xk_vm_load(xk_model *m, int32_t which, const xk_vm_ins *code, int32_t ncode,
                           const uint64_t *consts, int32_t nconsts, int32_t nregs)
 {
@@ -1431,8 +1461,12 @@ extern "C" int xk_vm_load(xk_model *m, int32_t which, const xk_vm_ins *code, int
                    "xk_vm_load: instruction %d (opcode %d) is malformed", pc, code[pc].op);
     if (m->vm_code[which]) cudaFree(m->vm_code[which]);
     if (m->vm_consts[which]) cudaFree(m->vm_consts[which]);
+    if (m->vm_ncodes[which]) cudaFree(m->vm_ncodes[which]);
+    if (m->vm_nconsts[which]) cudaFree(m->vm_nconsts[which]);
     m->vm_code[which] = nullptr;
     m->vm_consts[which] = nullptr;
+    m->vm_ncodes[which] = m->vm_nconsts[which] = nullptr;
+    m->vm_is_narrow[which] = false;
     m->vm_ncode[which] = 0;
     if (ncode > 0) {
         XK_CUDA(cudaMalloc(&m->vm_code[which], (size_t)ncode * sizeof(xk_vm_ins)));
@@ -1444,6 +1478,21 @@ extern "C" int xk_vm_load(xk_model *m, int32_t which, const xk_vm_ins *code, int
                             cudaMemcpyHostToDevice, m->stream));
     XK_CUDA(cudaStreamSynchronize(m->stream));
     m->vm_ncode[which] = ncode;
+    // the same program on 32-bit values, where it has that form
+    XkVmNarrow &v = m->vm_narrow[which];
+    if (xk_vm_translate(code, ncode, consts, nregs, m->vg, &v)) {
+        XK_CUDA(cudaMalloc(&m->vm_ncodes[which], v.code.size() * sizeof(uint32_t)));
+        XK_CUDA(cudaMemcpyAsync(m->vm_ncodes[which], v.code.data(), v.code.size() * sizeof(uint32_t),
+                                cudaMemcpyHostToDevice, m->stream));
+        if (!v.consts.empty()) {
+            XK_CUDA(cudaMalloc(&m->vm_nconsts[which], v.consts.size() * sizeof(uint32_t)));
+            XK_CUDA(cudaMemcpyAsync(m->vm_nconsts[which], v.consts.data(), v.consts.size() * sizeof(uint32_t),
+                                    cudaMemcpyHostToDevice, m->stream));
+        }
+        XK_CUDA(cudaStreamSynchronize(m->stream));
+        m->vm_is_narrow[which] = true;
+    }
+    m->vm_params_fit = vm_params_fit(m);
     return XK_OK;
 }
 
@@ -1457,5 +1506,7 @@ extern "C" int xk_vm_set_params(xk_model *m, const uint64_t *values, int32_t cou
     XK_CUDA(cudaMemcpyAsync(m->vm_params, values, (size_t)count * sizeof(uint64_t),
                             cudaMemcpyHostToDevice, m->stream));
     XK_CUDA(cudaStreamSynchronize(m->stream));
+    memcpy(m->vm_bound, values, (size_t)count * sizeof(uint64_t));
+    m->vm_params_fit = vm_params_fit(m);
     return XK_OK;
 }

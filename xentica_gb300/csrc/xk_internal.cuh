@@ -8,6 +8,7 @@
 #include <stdint.h>
 #include <stdio.h>
 #include <string>
+#include <vector>
 
 #include "../../include/xk.h"
 
@@ -278,6 +279,27 @@ struct VmGeo {
 cudaError_t xk_vm_run(const xk_vm_ins *code, int ncode, const uint64_t *consts,
                       const uint64_t *params, uint8_t *fld, int32_t *col, const VmGeo &g,
                       cudaStream_t s);
+
+// Programs whose values fit 32 bits (vm_narrow.cu): the translation of a
+// checked program (false: vm.cu runs it), and one pass of it.  Parameters are
+// taken as 32-bit values: each used slot's image must be the sign (sign) or
+// zero extension of its low half.  frame (a program that colours): also write
+// the zoom-1 frame of a 2-D lattice.
+struct XkVmParamUse {
+    uint16_t slot;
+    bool sign;
+};
+struct XkVmNarrow {
+    std::vector<uint32_t> code, consts;
+    std::vector<XkVmParamUse> params;
+    int nloads = 0, nops = 0, nslots = 0, colors = 0;
+    int threads = 0, smem = 0;   // of a block
+};
+bool xk_vm_translate(const xk_vm_ins *code, int ncode, const uint64_t *consts, int nregs, const VmGeo &g,
+                     XkVmNarrow *out);
+cudaError_t xk_vm_run_narrow(const XkVmNarrow &v, const uint32_t *code, const uint32_t *consts,
+                             const uint64_t *params, uint8_t *fld, int32_t *col, const VmGeo &g, cudaStream_t s,
+                             uint8_t *frame = nullptr, int frame_smooth = 0);
 
 // EvoLife family (evolife.cu)
 cudaError_t xk_evolife_set_positional(const double *lut54);
