@@ -145,3 +145,13 @@ def test_plan_cache_round_trip(monkeypatch, tmp_path):
     assert stored == [first.gpu.plan]
     got, want = _run(shape, "torus", 23, 5)
     assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("border", ["torus", "static1"])
+@pytest.mark.parametrize("shape", [(64, 1), (65, 3), (960, 16), (961, 1251), (1000, 1200), (2000, 3000), (3000, 4000)])
+def test_every_tile_height(shape, border, monkeypatch):
+    """Lattices whose tiles take each height, narrower and lower than a tile,
+    and words that straddle the wrap."""
+    monkeypatch.setenv("XK_TB", "8")
+    got, want = _run(shape, border, 11, 3)
+    assert np.array_equal(got, want)
