@@ -130,3 +130,43 @@ def test_long_run_and_tuner_choice(monkeypatch):
     fld = topo.field(cells, np.uint8)
     O.life_run(topo, fld, np.zeros(3 * n, np.int32), 1000)
     assert np.array_equal(model.gpu.arrays.cells.get()[:n], fld[:n])
+
+
+DEEP_SIZES = [(512, 512), (33, 40), (1024, 130), (100, 301), (1000, 700), (31, 16), (640, 360)]
+
+
+@pytest.mark.parametrize("band", [2, 3, 4, 6])
+@pytest.mark.parametrize("cluster", [2, 5, 16])
+@pytest.mark.parametrize("cls", [GameOfLife, GameOfLifeStatic])
+def test_rows_exchanged_every_8_generations(cls, cluster, band):
+    """The deep plan for every band length: slabs of 8 rows and more, a last
+    slab that is smaller, generation counts around the exchange period, odd
+    word counts and partial words; plans that do not apply are refused."""
+    import ctypes
+    from xentica_gb300 import _native as nat
+    for k, size in enumerate(DEEP_SIZES):
+        model = cls(type("E", (SoupExperiment, ), {"size": size}))
+        n = model.cells_num
+        cells = (np.random.RandomState(cluster + k).random_sample(n) < 0.45).astype(np.uint8)
+        model.gpu.load(cells, np.zeros(3 * n, dtype=np.int32))
+        model.gpu._ensure()
+        model.gpu._planned = True
+        plan = (ctypes.c_int32 * 4)(4, cluster, band, 0)
+        rc = model.gpu._lib.xk_model_set_plan(model.gpu._handle, plan)
+        rows = -(-size[1] // cluster)
+        slabs = -(-size[1] // rows)
+        lanes = 1 << (-(-size[0] // 32) - 1).bit_length()
+        warps = -(--(-(rows + 16) // band) // (32 // lanes))
+        fits = slabs >= 2 and size[1] - (slabs - 1) * rows >= 8 and warps <= 32
+        assert (rc == 0) == fits, (size, cluster, band)
+        if not fits:
+            continue
+        out = (ctypes.c_int32 * 4)()
+        nat.check(model.gpu._lib.xk_model_plan(model.gpu._handle, out), "xk_model_plan")
+        assert list(out) == [4, cluster, band, 0]
+        topo = O.Topology(size, "moore", 1 if cls is GameOfLifeStatic else None)
+        fld = topo.field(cells, np.uint8)
+        for gens in (1, 7, 8, 9, 16, 43):
+            model.gpu.step(gens)
+            O.life_run(topo, fld, np.zeros(3 * n, np.int32), gens)
+            assert np.array_equal(model.gpu.arrays.cells.get()[:n], fld[:n]), (size, cluster, band, gens)

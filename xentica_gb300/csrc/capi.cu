@@ -185,6 +185,10 @@ struct xk_model {
     int cl_tuned = 0, cl_C = 0, cl_R = 0, cl_threads = 0;   // cluster plan (cl_C = 0: none)
     int cl_want = 0, cl_band = 0;    // the cluster size and band length the plan was made from
     int cl_sync = 0;                 // the cluster plan's synchronisation form (XK_SYNC_*)
+    DeepPlan deep;                   // the plan with rows exchanged every 8 generations (deep.C = 0: none)
+    int deep_want = 0;               // the cluster size it was made from
+    unsigned int *gave_up = nullptr; // device: a bounded wait of its kernel gave up
+    bool cl_waits = false, deep_waits = false;   // kernels with bounded waits ran since the last download
     int tb_T = 0;                // temporally blocked global kernel: generations per launch (0: none)
     uint32_t rule0 = 0, rule1 = 0;
     int32_t lut[6] = {0, 0, 0, 0, 0, 0};
@@ -261,11 +265,23 @@ static int resident_plan_for(xk_model *m)
     return xk_life_resident_config(m->lg.W, m->lg.H, 8, &m->res_threads, &m->res_smem);
 }
 
+// whether a bounded wait of the model's deep cluster kernel gave up (clears it)
+static bool deep_gave_up(xk_model *m)
+{
+    unsigned int v = 0;
+    if (cudaMemcpyAsync(&v, m->gave_up, sizeof(v), cudaMemcpyDeviceToHost, m->stream) != cudaSuccess ||
+        cudaStreamSynchronize(m->stream) != cudaSuccess)
+        return false;
+    if (v) cudaMemsetAsync(m->gave_up, 0, sizeof(v), m->stream);
+    return v != 0;
+}
+
 // Multi-generation steps of a 2-D lattice run in one launch on the resident
 // kernel (one CTA) or on a cluster of 2..16 CTAs (cluster.cu).  On the first
 // such step the candidates (cluster sizes, and bands of 1, 2 or 4 rows per
 // lane group) are timed over 32 generations on the ping-pong partner buffer
-// (the state is not touched) and the fastest is kept; lattices too large for
+// (the state is not touched), then clusters that exchange rows every 8
+// generations (cluster_deep.cu), and the fastest is kept; lattices too large for
 // one CTA take the fastest cluster that fits, else the per-generation global
 // kernel.  XK_CLUSTER=0 disables clusters and XK_CLUSTER=n asks for a cluster
 // of (up to) n CTAs, with bands of XK_CLUSTER_BAND rows (default 2).
@@ -274,6 +290,7 @@ static int tune_cluster(xk_model *m)
     m->cl_tuned = 1;
     m->cl_C = 0;
     m->cl_sync = 0;
+    m->deep.C = 0;
     m->tb_T = 0;
     const char *tenv = getenv("XK_TB");
     if (tenv && tenv[0]) {
@@ -390,6 +407,28 @@ static int tune_cluster(xk_model *m)
             m->tb_T = 0;
         }
     }
+    // clusters that exchange rows every 8 generations
+    static const int deep_bands[] = {2, 3, 4, 6};
+    for (int want : cand)
+        for (int band : deep_bands) {
+            DeepPlan p;
+            if (!xk_life_deep_config(m->lg, want, band, &p)) continue;
+            float ms = 0.f;
+            XK_CUDA(time_it([&]() {
+                return xk_life_step_deep(scratch, m->lg, m->rule0, m->rule1, G, p, m->gave_up, m->stream);
+            }, &ms));
+            if (deep_gave_up(m)) {
+                xk_set_error("cluster step: a CTA gave up waiting for its neighbours' rows");
+                return XK_ERR_TIMEOUT;
+            }
+            if (ms < best) {
+                best = ms;
+                m->deep = p;
+                m->deep_want = want;
+                m->cl_C = 0;
+                m->tb_T = 0;
+            }
+        }
     return XK_OK;
 }
 
@@ -425,6 +464,7 @@ static void free_model(xk_model *m)
     }
     if (m->copy_stream) cudaStreamDestroy(m->copy_stream);
     if (m->d_inst) cudaFree(m->d_inst);
+    if (m->gave_up) cudaFree(m->gave_up);
     if (m->ev0) cudaEventDestroy(m->ev0);
     if (m->ev1) cudaEventDestroy(m->ev1);
     if (m->stream) cudaStreamDestroy(m->stream);
@@ -575,6 +615,8 @@ extern "C" int xk_model_create(const xk_desc *desc, xk_model **out)
             XK_TRY(cudaMalloc(&m->bits[1], (words + 4) * 4));
             XK_TRY(cudaMemsetAsync(m->bits[0], 0, (words + 4) * 4, m->stream));
             XK_TRY(cudaMalloc(&m->d_inst, sizeof(LifeInst)));
+            XK_TRY(cudaMalloc(&m->gave_up, sizeof(unsigned int)));
+            XK_TRY(cudaMemsetAsync(m->gave_up, 0, sizeof(unsigned int), m->stream));
             m->resident = resident_plan_for(m);
         } else {
             m->layout = LAYOUT_BYTES;
@@ -715,9 +757,11 @@ extern "C" int xk_download(xk_model *m, void *host_main, int64_t ncells)
     XK_CUDA(cudaMemcpyAsync(host_main, m->stage, (size_t)m->n * esz, cudaMemcpyDeviceToHost,
                             m->stream));
     XK_CUDA(cudaStreamSynchronize(m->stream));
-    // the neighbour form of the cluster kernel records bounded waits that
-    // gave up; the steps do not synchronise, so it is checked here
-    if (m->layout == LAYOUT_BITS2D && xk_cluster_take_wait_failure()) {
+    // the cluster kernels record bounded waits that gave up; the steps do not
+    // synchronise, so it is checked here
+    const bool gave_up = (m->deep_waits && deep_gave_up(m)) || (m->cl_waits && xk_cluster_take_wait_failure());
+    m->deep_waits = m->cl_waits = false;
+    if (gave_up) {
         xk_set_error("cluster step: a CTA gave up waiting for its neighbours' rows; the cells are "
                      "not valid");
         return XK_ERR_TIMEOUT;
@@ -943,10 +987,17 @@ static int step_enqueue(xk_model *m, int64_t first, int64_t count, uint8_t *fram
         return XK_OK;
     }
     const bool colors_free = colors_free_of(m);
-    if (m->layout == LAYOUT_BITS2D && colors_free && m->cl_C) {
+    if (m->layout == LAYOUT_BITS2D && colors_free && m->deep.C) {
+        // the same on clusters that exchange rows every 8 generations
+        m->deep_waits = true;
+        for (int64_t left = count; left > 0; left -= 4096)
+            XK_CUDA(xk_life_step_deep(m->bits[m->cur], m->lg, m->rule0, m->rule1,
+                                      (int)std::min<int64_t>(left, 4096), m->deep, m->gave_up, m->stream));
+    } else if (m->layout == LAYOUT_BITS2D && colors_free && m->cl_C) {
         // whole lattice in the shared memory of a cluster; long runs are cut
         // into launches of at most 4096 generations
         int64_t left = count;
+        m->cl_waits = m->cl_waits || m->cl_sync == XK_SYNC_NEIGHBOUR || m->cl_sync == XK_SYNC_ASYNC;
         while (left > 0) {
             const int g = (int)(left > 4096 ? 4096 : left);
             XK_CUDA(xk_life_step_cluster(m->bits[m->cur], m->lg, m->rule0, m->rule1, g, m->cl_C, m->cl_R,
@@ -1088,7 +1139,12 @@ extern "C" int xk_model_plan(xk_model *m, int32_t plan[4])
         int rc = tune_cluster(m);
         if (rc != XK_OK) return rc;
     }
-    if (m->cl_C) {
+    if (m->deep.C) {
+        plan[0] = XK_PLAN_DEEP;
+        plan[1] = m->deep_want;
+        plan[2] = m->deep.B;
+        plan[3] = 0;
+    } else if (m->cl_C) {
         plan[0] = XK_PLAN_CLUSTER;
         plan[1] = m->cl_want;
         plan[2] = m->cl_band;
@@ -1117,6 +1173,7 @@ extern "C" int xk_model_set_plan(xk_model *m, const int32_t plan[4])
                "xk_model_set_plan: only 2-D Life-like models with colours implied by the state "
                "have launch plans");
     int C = 0, R = 0, th = 0;
+    DeepPlan deep;
     switch (plan[0]) {
     case XK_PLAN_GLOBAL:
         XK_REQUIRE(!m->resident, XK_ERR_ARG, "xk_model_set_plan: this lattice fits one CTA");
@@ -1139,10 +1196,17 @@ extern "C" int xk_model_set_plan(xk_model *m, const int32_t plan[4])
         XK_REQUIRE(plan[3] >= 2 && plan[3] <= 8 && xk_life_tb_supported(m->lg), XK_ERR_ARG,
                    "xk_model_set_plan: temporal depth %d (2..8, width >= 64)", plan[3]);
         break;
+    case XK_PLAN_DEEP:
+        XK_REQUIRE(plan[1] >= 1 && plan[1] <= 16 && xk_life_deep_config(m->lg, plan[1], plan[2], &deep), XK_ERR_ARG,
+                   "xk_model_set_plan: no cluster of %d CTAs with %d rows a lane group that exchanges rows "
+                   "every 8 generations", plan[1], plan[2]);
+        break;
     default:
         XK_REQUIRE(false, XK_ERR_ARG, "xk_model_set_plan: unknown plan kind %d", plan[0]);
     }
     m->cl_tuned = 1;
+    m->deep = deep;
+    m->deep_want = plan[1];
     m->cl_C = C;
     m->cl_R = R;
     m->cl_threads = th;

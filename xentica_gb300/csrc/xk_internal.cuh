@@ -198,6 +198,17 @@ int xk_life_cluster_has_sync(const LifeGeo &g, int C, int R, int threads, int sy
 // a CTA of the neighbour form gave up waiting since the last call (clears it)
 bool xk_cluster_take_wait_failure();
 
+// The same lattices with rows exchanged every 8 generations
+// (cluster_deep.cu): config returns 0 where no cluster of (up to) C CTAs with
+// B (2, 3, 4, 6) rows a lane group applies (every CTA needs 8 rows); *gave_up
+// (device memory) is or-ed with 1 when a bounded wait gave up.
+struct DeepPlan {
+    int C = 0, R = 0, B = 0, bands = 0, threads = 0, smem = 0;
+};
+int xk_life_deep_config(const LifeGeo &g, int C, int B, DeepPlan *out);
+cudaError_t xk_life_step_deep(uint32_t *bits, const LifeGeo &g, uint32_t rule0, uint32_t rule1, int generations,
+                              const DeepPlan &p, unsigned int *gave_up, cudaStream_t s);
+
 // T (1..8) generations per launch of a 2-D lattice of any size (W >= 64),
 // tiles with a T-generation halo in shared memory, src -> dst (life_tb.cu)
 int xk_life_tb_supported(const LifeGeo &g);

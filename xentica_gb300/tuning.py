@@ -182,7 +182,7 @@ def tuned_band(lib, handle, widths, heights, generations, cache=True, library=No
     return int(chosen.value)
 
 
-PLAN_KINDS = {0: "global", 1: "resident", 2: "cluster", 3: "temporal"}
+PLAN_KINDS = {0: "global", 1: "resident", 2: "cluster", 3: "temporal", 4: "deep"}
 
 
 def lattice_key(device, library, width, height, border, rule_form=0):
