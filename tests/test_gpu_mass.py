@@ -188,3 +188,35 @@ def test_odd_widths_vs_oracle(size, form, monkeypatch):
     fld = topo.field(cells, np.uint32)
     O.mass_run(topo, fld, np.zeros(3 * n, dtype=np.int32), 1)
     assert np.array_equal(model.gpu.arrays.cells.get()[:n], fld[:n])
+
+
+@pytest.mark.parametrize("zc", ["", "1", "3", "7"])
+@pytest.mark.parametrize("size", [(1, 1, 2), (3, 2, 1), (5, 3, 9), (4, 4, 4), (129, 5, 6), (130, 33, 5), (128, 7, 8),
+                                  (255, 18, 7)])
+def test_small_totals_and_their_frames_vs_oracle(size, zc, monkeypatch):
+    """The kernel of totals below 2^30: row groups that end past the last row,
+    quads that end past the row, runs of one plane and of more planes than
+    there are, one cell holding nearly the whole allowed total; the same
+    generations with a frame each."""
+    if zc:
+        monkeypatch.setenv("XK_MASS_ZC", zc)
+    a, b = _model(size), _model(size)
+    n = a.cells_num
+    rng = np.random.RandomState(sum(size))
+    cells = rng.poisson(5, n).astype(np.uint32)
+    cells[n // 2] = 0
+    cells[n // 2] = 2 ** 30 - 1 - int(cells.sum())
+    for m in (a, b):
+        m.gpu.load(cells, np.zeros(3 * n, dtype=np.int32))
+    topo = _topo(size)
+    fld, col, totals = topo.field(cells, np.uint32), np.zeros(3 * n, dtype=np.int32), []
+    b.set_viewport(size[:2])
+    frames = b.step_frames(5)
+    a.gpu.step(5)
+    for g in range(5):
+        O.mass_run(topo, fld, col, 1, totals=totals)
+        want = O.render(topo, col, size[0], size[1]).astype(np.uint8)
+        assert np.array_equal(frames[g], want.ravel()), g
+    for m in (a, b):
+        assert np.array_equal(m.gpu.arrays.cells.get()[:n], fld[:n])
+        assert m.gpu.mass_totals(5).tolist() == totals

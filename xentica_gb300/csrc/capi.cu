@@ -585,7 +585,7 @@ extern "C" int xk_model_create(const xk_desc *desc, xk_model **out)
             XK_TRY(cudaMalloc(&m->cells32[1], bytes));
             XK_TRY(cudaMemsetAsync(m->cells32[0], 0, bytes, m->stream));
             XK_TRY(cudaMemsetAsync(m->cells32[1], 0, bytes, m->stream));
-            XK_TRY(cudaMalloc(&m->proj, (size_t)d.size[0] * d.size[1] * 4));
+            XK_TRY(cudaMalloc(&m->proj, (size_t)xk_mass_pitch(d.size[0]) * d.size[1] * 4));
         } else if (d.family == XK_FAMILY_NOISE) {
             m->layout = LAYOUT_NOISE;
             XK_TRY(cudaMalloc(&m->cells16, (size_t)n * 2));
@@ -1266,7 +1266,7 @@ static int render_enqueue(xk_model *m, void *img, bool bytes, int32_t width, int
 // the loop.  Host frames go through the device ring as in xk_step_frames.
 static int mass_frames_enqueue(xk_model *m, int64_t nsteps, uint8_t *frames, bool on_device, size_t fb)
 {
-    const size_t pbytes = (size_t)m->d.size[0] * m->d.size[1] * 4;
+    const size_t pbytes = (size_t)xk_mass_pitch(m->d.size[0]) * m->d.size[1] * 4;
     if (!m->proj2) XK_CUDA(cudaMalloc(&m->proj2, pbytes));
     uint32_t *P[2] = {m->proj, m->proj2};
     XK_CUDA(cudaMemsetAsync(P[0], 0, pbytes, m->stream));
@@ -1354,7 +1354,7 @@ extern "C" int xk_step_frames(xk_model *m, int64_t nsteps, int32_t width, int32_
     // column colours as it writes the cells (no second pass over the state)
     const bool mass_fused = m->layout == LAYOUT_MASS && m->d.proj_axis0 == 0 && m->d.proj_axis1 == 1 &&
                             m->d.render_smooth == 0 && zoom == 1 && dx == 0 && dy == 0 &&
-                            width == m->d.size[0] && height == m->d.size[1] && xk_mass_fuses_projection(m->d);
+                            width == m->d.size[0] && height == m->d.size[1] && xk_mass_fuses_projection(m->d, m->mass_small);
     XK_CUDA(cudaEventRecord(m->ev0, m->stream));
     if (mass_fused) {
         rc = mass_frames_enqueue(m, nsteps, frames, frames_on_device != 0, fb);

@@ -11,10 +11,10 @@
 //   m'         = m - sum_k sent_k + sum_k incoming_k
 // Colour (plain ColorEffect): min(m' * 32, 255) on every channel.
 //
-// Three kernels: xk_k_mass_tma (tensor copies into a shared-memory ring,
-// widths that are a multiple of 4: the default), xk_k_mass_rows (the same
-// widths, register queue and plain loads; XK_MASS_KERNEL=rows) and the
-// generic xk_k_mass for any width.  Work split of the generic one: a
+// Kernels: mass_quads.cu's where the total is below 2^30; xk_k_mass_tma (tensor
+// copies into a shared-memory ring) for the rest; with XK_MASS_KERNEL=rows
+// xk_k_mass_rows (register queue and plain loads, widths that are a multiple
+// of 4) and the generic xk_k_mass for any width.  Work split of the generic one: a
 // CTA owns a 32-wide, 8-row tile of a run of zc planes; a thread owns one
 // cell of a row and walks its z run with a three-plane register queue.
 // x neighbours come from the neighbouring lanes (shuffles; lanes 0 and 31
@@ -35,7 +35,6 @@
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
-#include <type_traits>
 
 #include "xk_internal.cuh"
 
@@ -424,10 +423,9 @@ xk_k_mass_rows(const uint32_t *__restrict__ src, uint32_t *__restrict__ dst,
 // the plane's tile or halo is at or above 2^30 (so the one-instruction q may
 // be inexact, or a wall value is inside).  A plane whose tile saw such a
 // cell in planes z - 1 .. z + 1 takes the exact per-neighbour form for the
-// whole CTA, reading the neighbours from global memory.  When the uploaded
-// lattice's total mass is below 2^30, no cell can ever reach 2^30 (mass is
-// conserved and never negative) and the fast-only instantiation runs: plain
-// barriers, no flag and no exact path, so fewer registers.
+// whole CTA, reading the neighbours from global memory.  (A lattice whose
+// total mass is below 2^30 never holds such a cell and runs on
+// mass_quads.cu's kernel.)
 #define XK_MT_BY 8
 #define XK_MT_STAGES 4
 #define XK_MT_COLS 136                                  // 4 + 128 + 4
@@ -483,15 +481,6 @@ __device__ __forceinline__ void xk_mt_issue(const CUtensorMap *tm, uint32_t stag
                  : "memory");
 }
 
-// the barrier of a plane; the general kernel also ORs the flags of its threads
-template <bool GENERAL>
-__device__ __forceinline__ bool xk_mt_barrier(bool flag)
-{
-    if (GENERAL) return __syncthreads_or(flag);
-    __syncthreads();
-    return false;
-}
-
 // q of four cells, and whether one of them is at or above 2^30
 __device__ __forceinline__ uint4 xk_mt_q4(const uint4 m, bool &big)
 {
@@ -500,7 +489,7 @@ __device__ __forceinline__ uint4 xk_mt_q4(const uint4 m, bool &big)
 }
 
 // PROJ: also add the colours of the cells it writes, per column, into
-// proj[y * W + x] (the z-projection RendererPlain renders; proj zeroed
+// proj[y * P + x] (the z-projection RendererPlain renders; proj zeroed
 // before the launch): a thread sums its four columns over its run of planes
 // (two columns per register, 16 bits each: a colour is at most 255 and a run
 // at most 256 planes, which the host checks) and adds each sum with one
@@ -514,7 +503,7 @@ __device__ __forceinline__ uint4 xk_mt_q4(const uint4 m, bool &big)
 // RendererPlain renders it at zoom 1, and zero the column for the generation
 // after this one (the sums alternate between two buffers).  So a frame every
 // generation adds no launch between two generations.
-template <int MINB, bool GENERAL, bool PROJ>
+template <int MINB, bool PROJ>
 __global__ void __launch_bounds__(32 * XK_MT_BY, MINB)
 xk_k_mass_tma(const __grid_constant__ CUtensorMap tm, const uint32_t *__restrict__ src,
               uint32_t *__restrict__ dst, unsigned long long *__restrict__ total, MassParams p, int zc,
@@ -558,12 +547,12 @@ xk_k_mass_tma(const __grid_constant__ CUtensorMap tm, const uint32_t *__restrict
     if (PROJ && frame_prev && blockIdx.z == 0 && in) {
         // the previous generation's frame from its column sums (this
         // thread's four columns), and those sums zeroed for the next one
-        const int64_t c0 = (int64_t)y * p.W + x0;
+        const int64_t c0 = (int64_t)y * p.P + x0, f0 = (int64_t)y * p.W + x0;
 #pragma unroll
         for (int i = 0; i < 4; ++i)
             if (x0 + i < p.W) {
                 const uint8_t v = (uint8_t)(int)__fdiv_rn((float)proj_prev[c0 + i], (float)p.D);
-                uint8_t *px = frame_prev + 3 * (c0 + i);
+                uint8_t *px = frame_prev + 3 * (f0 + i);
                 px[0] = v;
                 px[1] = v;
                 px[2] = v;
@@ -629,14 +618,14 @@ xk_k_mass_tma(const __grid_constant__ CUtensorMap tm, const uint32_t *__restrict
     uint4 m0, q0, m1, q1, m2, q2;
     bool b_prev = false, b_cur = false;
     take(nullptr, m0, q0, b_prev);                    // plane z0 - 1: q of the own column
-    b_prev = xk_mt_barrier<GENERAL>(b_prev);
+    b_prev = __syncthreads_or(b_prev);
     if (*fail) {
         if (tid == 0) atomicOr(&xk_mass_wait_failed, 1u);
         return;
     }
     advance();
     take(qt0, m1, q1, b_cur);                         // plane z0
-    b_cur = xk_mt_barrier<GENERAL>(b_cur);
+    b_cur = __syncthreads_or(b_cur);
     if (*fail) {
         if (tid == 0) atomicOr(&xk_mass_wait_failed, 1u);
         return;
@@ -650,9 +639,7 @@ xk_k_mass_tma(const __grid_constant__ CUtensorMap tm, const uint32_t *__restrict
     const uint32_t c2 = cy + 1 + (x0 + 3 < p.W), c3 = cy + 1 + (x0 + 4 < p.W);
     // cells at or beyond W (padding) are written as 0
     const bool v1 = x0 + 1 < p.W, v2 = x0 + 2 < p.W, v3 = x0 + 3 < p.W;
-    // the fast-only form runs when the lattice's whole total is below 2^30,
-    // so every partial sum of its cells fits 32 bits
-    typename std::conditional<GENERAL, unsigned long long, uint32_t>::type mass_sum = 0;
+    unsigned long long mass_sum = 0;
     uint32_t cs01 = 0u, cs23 = 0u;                   // PROJ: colour sums, two columns per word
     uint32_t off = in ? (uint32_t)z0 * plane + (uint32_t)y * p.P + x0 : 0u;
     int z = z0;
@@ -662,12 +649,12 @@ xk_k_mass_tma(const __grid_constant__ CUtensorMap tm, const uint32_t *__restrict
                     const uint32_t *qcur, uint32_t *qnext) -> bool {
         bool b_t = false;
         take(qnext, mn, qn, b_t);
-        const bool b_next = xk_mt_barrier<GENERAL>(b_t);
+        const bool b_next = __syncthreads_or(b_t);
         if (*fail) return false;
         advance();
         const uint32_t cz = (uint32_t)((z > 0) + (z + 1 < p.D));
         uint32_t out[4];
-        if (!GENERAL || !(b_prev | b_cur | b_next)) {
+        if (!(b_prev | b_cur | b_next)) {
             const uint4 up = *reinterpret_cast<const uint4 *>(qcur + own - XK_MT_COLS);
             const uint4 dn = *reinterpret_cast<const uint4 *>(qcur + own + XK_MT_COLS);
             const uint32_t hl = qcur[own - 1], hr = qcur[own + 4];
@@ -678,7 +665,7 @@ xk_k_mass_tma(const __grid_constant__ CUtensorMap tm, const uint32_t *__restrict
             out[1] = mc.y - qc.y * (c1 + cz) + qc.x + qc.z + up.y + dn.y + qp.y + qn.y;
             out[2] = mc.z - qc.z * (c2 + cz) + qc.y + qc.w + up.z + dn.z + qp.z + qn.z;
             out[3] = mc.w - qc.w * (c3 + cz) + qc.z + xr + up.w + dn.w + qp.w + qn.w;
-        } else if (GENERAL && in) {
+        } else if (in) {
             // the reference's arithmetic per neighbour, neighbours from global memory
             const uint32_t wall = p.wall;
 #pragma unroll
@@ -702,10 +689,7 @@ xk_k_mass_tma(const __grid_constant__ CUtensorMap tm, const uint32_t *__restrict
         out[3] = v3 ? out[3] : 0u;
         if (in) {
             *reinterpret_cast<uint4 *>(dst + off) = make_uint4(out[0], out[1], out[2], out[3]);
-            if (GENERAL)
-                mass_sum += (unsigned long long)out[0] + out[1] + (unsigned long long)out[2] + out[3];
-            else
-                mass_sum += out[0] + out[1] + out[2] + out[3];
+            mass_sum += (unsigned long long)out[0] + out[1] + (unsigned long long)out[2] + out[3];
             if (PROJ) {
                 cs01 += xk_mass_color(out[0]) + (xk_mass_color(out[1]) << 16);
                 cs23 += xk_mass_color(out[2]) + (xk_mass_color(out[3]) << 16);
@@ -726,7 +710,7 @@ xk_k_mass_tma(const __grid_constant__ CUtensorMap tm, const uint32_t *__restrict
         return;
     }
     if (PROJ && in) {
-        uint32_t *pc = proj + (int64_t)y * p.W + x0;
+        uint32_t *pc = proj + (int64_t)y * p.P + x0;
         const uint32_t csum[4] = {cs01 & 0xFFFFu, cs01 >> 16, cs23 & 0xFFFFu, cs23 >> 16};
 #pragma unroll
         for (int i = 0; i < 4; ++i)
@@ -742,7 +726,7 @@ xk_k_mass_tma(const __grid_constant__ CUtensorMap tm, const uint32_t *__restrict
     }
 }
 
-// column colour sums of a state (pitched rows; the sums are W * H, unpadded).
+// column colour sums of a state (rows of the sums at the state's pitch).
 // A CTA owns 32 columns of one row y: its 8 warps take every 8th plane each
 // (a warp reads 32 consecutive cells of a plane row, 128 bytes), four loads
 // in flight per thread, and the 8 partial sums of a column meet in shared
@@ -778,7 +762,7 @@ xk_k_mass_project(const uint32_t *__restrict__ src, uint32_t *__restrict__ proj,
             uint32_t t = 0;
 #pragma unroll
             for (int k = 0; k < XK_PROJ_ZS; ++k) t += part[k][threadIdx.x];
-            proj[y * p.W + x] = t;
+            proj[y * p.P + x] = t;
             if (frame) {
                 const uint8_t v = (uint8_t)(int)__fdiv_rn((float)t, (float)p.D);
                 uint8_t *px = frame + 3 * (y * p.W + x);
@@ -822,7 +806,7 @@ __global__ void xk_k_mass_render(const uint32_t *__restrict__ proj, T *__restric
     if (xa >= p.W) xa = xa % p.W;
     if (xb < 0) xb = p.H - (-xb % p.H);
     if (xb >= p.H) xb = xb % p.H;
-    const float s = (float)proj[(int64_t)xb * p.W + xa];
+    const float s = (float)proj[(int64_t)xb * p.P + xa];
     const T v = (T)(int)__fdiv_rn(s, (float)p.D);
     img[3 * ip] = v;
     img[3 * ip + 1] = v;
@@ -895,9 +879,18 @@ static void mass_tma_shape(const MassParams &p, int *gx, int *gy, int *zc)
     if (!getenv("XK_MASS_ZC")) *zc = std::max(*zc, std::min(4, p.D));
 }
 
-bool xk_mass_fuses_projection(const xk_desc &d)
+// the fast-only kernel: the lattice's total is below 2^30 (XK_MASS_GENERAL=1
+// in the environment takes the general ones anyway)
+static bool mass_quads(const xk_desc &d, bool small)
+{
+    const char *g = getenv("XK_MASS_GENERAL");
+    return small && !(g && g[0] == '1') && xk_mass_quads_apply(d);
+}
+
+bool xk_mass_fuses_projection(const xk_desc &d, bool small)
 {
     if (!mass_tma_enabled()) return false;
+    if (mass_quads(d, small)) return xk_mass_quads_project(d);
     int gx, gy, zc;
     mass_tma_shape(mass_params(d), &gx, &gy, &zc);
     return zc <= 256;   // the 16-bit column sums of a run of planes
@@ -910,7 +903,7 @@ __global__ void xk_k_mass_frame(const uint32_t *__restrict__ proj, uint8_t *__re
 {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (int64_t)p.W * p.H) return;
-    const uint8_t v = (uint8_t)(int)__fdiv_rn((float)proj[i], (float)p.D);
+    const uint8_t v = (uint8_t)(int)__fdiv_rn((float)proj[i / p.W * p.P + i % p.W], (float)p.D);
     frame[3 * i] = v;
     frame[3 * i + 1] = v;
     frame[3 * i + 2] = v;
@@ -930,6 +923,8 @@ cudaError_t xk_mass_step(const uint32_t *src, uint32_t *dst, unsigned long long 
 {
     const MassParams p = mass_params(d);
     const bool vec = p.W % 4 == 0;
+    if (mass_tma_enabled() && mass_quads(d, small))
+        return xk_mass_step_quads(src, dst, total, d, s, proj, proj_prev, frame_prev);
     if (mass_tma_enabled()) {
         PFN_cuTensorMapEncodeTiled_v12000 enc = xk_tensor_map_encoder();
         if (!enc) return cudaErrorNotSupported;
@@ -948,28 +943,16 @@ cudaError_t xk_mass_step(const uint32_t *src, uint32_t *dst, unsigned long long 
         mass_tma_shape(p, &gx, &gy, &zc);
         dim3 block(32, XK_MT_BY);
         dim3 grid(gx, gy, (p.D + zc - 1) / zc);
-        // a lattice whose total mass is below 2^30 keeps every cell below 2^30
-        // (mass is conserved and never negative), so no cell can need the exact
-        // form and no wall value can be inside: the fast-only instantiation.
-        // XK_MASS_GENERAL=1 in the environment takes the general one anyway.
-        const char *g = getenv("XK_MASS_GENERAL");
-        const bool fast = small && !(g && g[0] == '1');
         // programmatic dependent launch: this generation's CTAs may start
         // their set-up while the previous generation's last CTAs run
         if (proj) {
             if (zc > 256) return cudaErrorNotSupported;   // the 16-bit column sums would overflow
-            if (fast)
-                return xk_launch_pdl(xk_k_mass_tma<4, false, true>, grid, block, XK_MT_SMEM, s, tm, src, dst, total,
-                                     p, zc, proj, proj_prev, frame_prev);
-            return xk_launch_pdl(xk_k_mass_tma<3, true, true>, grid, block, XK_MT_SMEM, s, tm, src, dst, total, p,
+            return xk_launch_pdl(xk_k_mass_tma<3, true>, grid, block, XK_MT_SMEM, s, tm, src, dst, total, p,
                                  zc, proj, proj_prev, frame_prev);
         }
         uint32_t *const none = nullptr;
         uint8_t *const no_frame = nullptr;
-        if (fast)
-            return xk_launch_pdl(xk_k_mass_tma<4, false, false>, grid, block, XK_MT_SMEM, s, tm, src, dst, total, p,
-                                 zc, none, none, no_frame);
-        return xk_launch_pdl(xk_k_mass_tma<4, true, false>, grid, block, XK_MT_SMEM, s, tm, src, dst, total, p, zc,
+        return xk_launch_pdl(xk_k_mass_tma<4, false>, grid, block, XK_MT_SMEM, s, tm, src, dst, total, p, zc,
                              none, none, no_frame);
     }
     if (proj) return cudaErrorNotSupported;   // the other forms write no projection
