@@ -106,3 +106,50 @@ def test_frames_vs_oracle_render():
         O.gravity_run(topo, fld, col, 1, color=O._color(True, 255, 255, 1))
         img = O.render(topo, col, size[0], size[1], smooth=1).astype(np.uint8)
         assert np.array_equal(frames[g], img), g
+
+
+# windows write 60 x 30 cells, four a thread: one to three cells over a
+# window or a quad, rows that start off a 16-byte boundary
+@pytest.mark.parametrize("size", [(4, 3), (59, 29), (60, 30), (61, 31), (62, 60), (63, 61), (64, 2), (120, 1),
+                                  (121, 91), (182, 59), (7, 32)])
+@pytest.mark.parametrize("cls,border", [(GraviCowboys, None), (GraviCowboysStatic, STATIC)])
+def test_window_edges_vs_oracle(cls, border, size):
+    """Cells, colours and frames at the edges of windows, quads and rows."""
+    n = size[0] * size[1]
+    cells = random_cells(n, n, energies=8)
+    _run(cls, border, size, cells, n, steps=(1, 3))
+    model, colors = _model(cls, size, cells, n)
+    model.set_viewport(size)
+    topo = O.Topology(size, "moore", border)
+    fld = topo.field(cells, np.uint64)
+    col = colors.copy()
+    frames = model.step_frames(4)
+    for g in range(4):
+        O.gravity_run(topo, fld, col, 1, color=O._color(True, 255, 255, 1))
+        img = O.render(topo, col, size[0], size[1], smooth=1).astype(np.uint8)
+        assert np.array_equal(frames[g], img), (size, g)
+
+
+@pytest.mark.parametrize("cls,border", [(GraviCowboys, None), (GraviCowboysStatic, STATIC)])
+def test_special_gravities_vs_oracle(cls, border):
+    """NaN, infinite and negative-zero gravities among ties: a comparison
+    with a NaN keeps the lowest so far, in neighbour order.  (A NaN's bits
+    are the processor's own: compared as NaN.)"""
+    size = (130, 67)
+    n = size[0] * size[1]
+    cells = random_cells(n, 3, energies=10)
+    rng = np.random.RandomState(4)
+    special = np.array([np.nan, np.inf, -np.inf, -0.0, 0.0], dtype=np.float32).view(np.uint32).astype(np.uint64)
+    pick = rng.randint(0, 5, n)
+    at = rng.random_sample(n) < 0.05
+    cells = np.where(at, (cells & np.uint64(0xFFFFFF)) | special[pick] << np.uint64(24), cells)
+    model, _ = _model(cls, size, cells, 3)
+    topo = O.Topology(size, "moore", border)
+    fld = topo.field(cells, np.uint64)
+    model.gpu.step(1)
+    O.gravity_run(topo, fld, np.zeros(3 * n, dtype=np.int32), 1)
+    got, want = model.gpu.arrays.cells.get()[:n], fld[:n]
+    assert np.array_equal(got & np.uint64(0xFFFFFF), want & np.uint64(0xFFFFFF))
+    g, w = [(a >> np.uint64(24)).astype(np.uint32).view(np.float32) for a in (got, want)]
+    assert np.isnan(w).any() and np.isinf(w).any()
+    assert np.array_equal(g, w, equal_nan=True)

@@ -48,11 +48,12 @@ __device__ __forceinline__ void xk_pack_px4(const uint32_t r[4], const uint32_t 
 // lies: a row of pixels starts at any byte of a frame.  At an offset of s
 // bytes from a word each lane writes its bytes after the s that belong to
 // its neighbour's last word; the ends go byte by byte.  The whole warp calls
-// it; lanes outside first .. last store nothing.
+// it (with one row of lanes, or several); lanes outside first .. last store
+// nothing.
 __device__ __forceinline__ void xk_store_px4(uint8_t *dst, const uint32_t w[3], int lane, int first, int last)
 {
-    const uint32_t s = (uint32_t)(uintptr_t)dst & 3u;       // the same in every lane
-    const uint32_t prev = s ? __shfl_up_sync(0xFFFFFFFFu, w[2], 1) : 0u;
+    const uint32_t s = (uint32_t)(uintptr_t)dst & 3u;       // the same in first .. last
+    const uint32_t prev = __shfl_up_sync(0xFFFFFFFFu, w[2], 1);
     if (lane < first || lane > last) return;
     uint32_t *a = (uint32_t *)(dst - s);
     if (s == 0) {
