@@ -105,3 +105,37 @@ def test_uniform_genomes_step_transitions_to_10000():
         _oracle_step(model, fld, col, 1)
         assert np.array_equal(model.gpu.arrays.cells.get()[:n], fld[:n]), "generation %d" % g
         assert np.array_equal(model.gpu.arrays.colors.get(), col), "colours, generation %d" % g
+
+
+# four cells a thread on tiles of 64 x 16 from 3 * 2^18 cells in rows of a
+# multiple of four; the others one a thread
+@pytest.mark.parametrize("size", [(1028, 769), (4100, 192), (1024, 768), (1020, 771), (1027, 769), (131, 103)])
+@pytest.mark.parametrize("legacy,mutation,live", [(True, 0.0, 0.6), (False, 0.2, 0.6), (True, 0.01, 0.05),
+                                                  (False, 0.0, 1.0)])
+def test_quads_vs_oracle(size, legacy, mutation, live):
+    """Cells, colours (negative ones too) and frames at the edges of tiles."""
+    w, h = size
+    n = w * h
+    model = _model(size, legacy, mutation_prob=mutation, death_speed=9, max_genes=7, fade_in=30, fade_out=7)
+    rng = np.random.RandomState(n + int(live * 100))
+    energy = rng.randint(0, 300, n).astype(np.uint64)
+    rule = rng.randint(0, 2 ** 18, n).astype(np.uint64) * (rng.random_sample(n) < live)
+    # a patch of few birth bits: ties of five to eight parents
+    rule[:n // 4] &= np.uint64(0x3FC81)
+    cells = energy + (rule << np.uint64(9)) + (rng.randint(0, 2 ** 16, n).astype(np.uint64) << np.uint64(27))
+    colors = rng.randint(-300, 300, 3 * n).astype(np.int32)
+    model.gpu.load(cells, colors)
+    model.set_viewport(size)
+    topo = O.Topology(size)
+    fld = topo.field(cells, np.uint64)
+    col = colors.copy()
+    frames = model.step_frames(3)
+    for g in range(3):
+        _oracle_step(model, fld, col, 1)
+        assert np.array_equal(frames[g], O.render(topo, col, w, h, smooth=1).astype(np.uint8)), g
+    assert np.array_equal(model.gpu.arrays.cells.get()[:n], fld[:n])
+    assert np.array_equal(model.gpu.arrays.colors.get(), col)
+    model.gpu.step(2)
+    _oracle_step(model, fld, col, 2)
+    assert np.array_equal(model.gpu.arrays.cells.get()[:n], fld[:n])
+    assert np.array_equal(model.gpu.arrays.colors.get(), col)

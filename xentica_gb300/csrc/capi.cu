@@ -951,7 +951,7 @@ static int step_enqueue(xk_model *m, int64_t first, int64_t count, uint8_t *fram
     if (m->layout == LAYOUT_CELLS64) {
         for (int64_t g = 0; g < count; ++g) {
             XK_CUDA(xk_evolife_step(m->cells64[m->cur], m->cells64[1 - m->cur], m->col, m->d,
-                                    m->mut_thresh, m->stream, frame, m->d.render_smooth));
+                                    m->mut_thresh, m->col_range, m->stream, frame, m->d.render_smooth));
             m->cur = 1 - m->cur;
         }
         return XK_OK;

@@ -23,7 +23,7 @@ static __device__ __noinline__ uint32_t xk_pixel(int c, int smooth)
     return (uint32_t)(int)f;
 }
 
-__device__ __forceinline__ bool xk_px_small(int c) { return (uint32_t)c + (1u << 24) < (1u << 25); }
+__host__ __device__ __forceinline__ bool xk_px_small(int c) { return (uint32_t)c + (1u << 24) < (1u << 25); }
 
 // Host: whether every colour that starts below 2^24 in magnitude keeps a
 // pixel equal to its low byte (a faded colour lies between the old one and
@@ -75,5 +75,147 @@ __device__ __forceinline__ void xk_store_px4(uint8_t *dst, const uint32_t w[3], 
         dst[11] = (uint8_t)(w[2] >> 24);
         if (s > 1u) dst[10] = (uint8_t)(w[2] >> 16);
         if (s > 2u) dst[9] = (uint8_t)(w[2] >> 8);
+    }
+}
+
+// The last 1 to 3 cells of a row, which xk_store_px4 leaves: their bytes
+__device__ __forceinline__ void xk_store_px_rest(uint8_t *at, const uint32_t w[3], int cells)
+{
+#pragma unroll
+    for (int k = 0; k < 9; ++k)
+        if (k < 3 * cells) at[k] = (uint8_t)(w[k >> 2] >> (8 * (k & 3)));
+}
+
+// The pixels' bytes of the four cells whose colours stand at mine, any
+// colours.  (One call out of line: inlined, or called per colour, its
+// registers cost the common path 8 %.)
+static __device__ __noinline__ uint3 xk_pixels4_any(const int *mine, int smooth)
+{
+    uint32_t b[3] = {0, 0, 0};
+#pragma unroll
+    for (int w = 0; w < 3; ++w)
+#pragma unroll 1
+        for (int k = 0; k < 4; ++k) {
+            float f = (float)mine[4 * w + k];
+            if (smooth > 0) f = __fdiv_rn(f, (float)smooth);
+            b[w] = b[w] >> 8 | (uint32_t)(int)f << 24;
+        }
+    return make_uint3(b[0], b[1], b[2]);
+}
+
+// Whether all twelve are below 2^24 in magnitude
+__device__ __forceinline__ bool xk_px_small12(const int c[12])
+{
+    int lo = min(c[0], c[1]), hi = max(c[0], c[1]);
+#pragma unroll
+    for (int k = 2; k < 12; k += 2) {
+        lo = __vimin3_s32(lo, c[k], c[k + 1]);
+        hi = __vimax3_s32(hi, c[k], c[k + 1]);
+    }
+    return xk_px_small(lo) && xk_px_small(hi);
+}
+
+// The pixels' bytes of four cells' colours c, which also stand at mine.
+// small: every pixel is its colour's low byte.
+__device__ __forceinline__ void xk_pixels4(const int c[12], const int *mine, bool small, int smooth, uint32_t b[3])
+{
+    uint32_t px[3][4];
+#pragma unroll
+    for (int k = 0; k < 12; ++k) px[k % 3][k / 3] = (uint32_t)c[k];
+    xk_pack_px4(px[0], px[1], px[2], b);
+    if (!small) {
+        const uint3 v = xk_pixels4_any(mine, smooth);
+        b[0] = v.x;
+        b[1] = v.y;
+        b[2] = v.z;
+    }
+}
+
+// ---------------------------------------------------------------------------
+// A row of colours through shared memory, by a half warp (lane q of 16) whose
+// lanes hold four cells each: global memory is read and written in the row's
+// 16-byte pieces in order (whole sectors a warp; a lane's own 48 bytes at 16
+// an access touch every sector three times), a lane's twelve words are read
+// and written in shared memory.  A row that starts off a 16-byte boundary
+// keeps its offset in its buffer; ALIGNED: W % 4 == 0, none does.
+
+// 16-byte pieces of a buffer for a row of this many cells
+__host__ __device__ constexpr int xk_col_pieces(int cells) { return cells / 4 * 3 + 1; }
+
+template <int BYTES>
+__device__ __forceinline__ void xk_copy_async(void *dst, const void *src)
+{
+    const uint32_t to = (uint32_t)__cvta_generic_to_shared(dst);
+    if (BYTES == 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to), "l"(src) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(to), "l"(src) : "memory");
+}
+
+// Starts the copy of `cells` cells' colours, the first word at col + first,
+// of a lattice of `words` colour words (cp.async.wait_all ends it)
+template <bool ALIGNED, int CELLS>
+__device__ __forceinline__ void xk_col_fetch(int4 *buf, const int32_t *col, int64_t first, int cells,
+                                             int64_t words, int q)
+{
+    const int off = ALIGNED ? 0 : (int)(first & 3);
+    const int *at = col + (first - off);
+    // pieces up to the row's end, whole ones up to the lattice's
+    const int end = off + 3 * cells;
+    const int full = ALIGNED ? end : min(end, (int)min(words - (first - off), (int64_t)(3 * CELLS + 12)) - 3);
+#pragma unroll
+    for (int k = q; k < (ALIGNED ? CELLS / 4 * 3 : xk_col_pieces(CELLS)); k += 16)
+        if (4 * k < full) xk_copy_async<16>(buf + k, at + 4 * k);
+    if (!ALIGNED && full < end) {       // the lattice's last words
+        const int k = (max(full, 0) + 3 & ~3) + q;
+        if (k < end) xk_copy_async<4>((int *)buf + k, at + k);
+    }
+}
+
+template <bool ALIGNED>
+__device__ __forceinline__ void xk_col_read(const int *mine, int c[12])
+{
+    if (ALIGNED) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const int4 o = ((const int4 *)mine)[k];
+            c[4 * k] = o.x;
+            c[4 * k + 1] = o.y;
+            c[4 * k + 2] = o.z;
+            c[4 * k + 3] = o.w;
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < 12; ++k) c[k] = mine[k];
+    }
+}
+
+template <bool ALIGNED>
+__device__ __forceinline__ void xk_col_write(int *mine, const int c[12])
+{
+    if (ALIGNED) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+            ((int4 *)mine)[k] = make_int4(c[4 * k], c[4 * k + 1], c[4 * k + 2], c[4 * k + 3]);
+    } else {
+#pragma unroll
+        for (int k = 0; k < 12; ++k) mine[k] = c[k];
+    }
+}
+
+// Stores a row that all its lanes have written (__syncwarp between)
+template <bool ALIGNED, int CELLS>
+__device__ __forceinline__ void xk_col_store(const int4 *buf, int32_t *col, int64_t first, int cells, int q)
+{
+    const int off = ALIGNED ? 0 : (int)(first & 3);
+    int *at = col + (first - off);
+    const int end = off + 3 * cells;
+#pragma unroll
+    for (int k = q; k < (ALIGNED ? CELLS / 4 * 3 : xk_col_pieces(CELLS)); k += 16)
+        if (4 * k >= off && 4 * k + 4 <= end) *(int4 *)(at + 4 * k) = buf[k];
+    if (!ALIGNED) {     // the first and last words: pieces shared with the cells beside
+        const int k = q < 4 ? q : (end & ~3) + q - 4;
+        if (q < 4 ? off > 0 && k >= off && k < end : q < 8 && k >= (off > 0 ? 4 : 0) && k < end)
+            at[k] = ((const int *)buf)[k];
     }
 }

@@ -30,9 +30,10 @@
 // state but a quotient outside the range of the float division.  Colours go
 // through shared memory: 48 bytes a lane, but whole sectors a warp both ways,
 // and on their way while the states are emitted (16-byte accesses of a lane's
-// own 48 bytes ran a generation in 19.0 us, this in 17.2).
+// own 48 bytes ran a generation in 19.0 us, this in 17.2, before the pixels of
+// colours beyond 2^24 moved out of line).
 //
-// 64 frames of 1920 x 1080: 1102 us, against 1412 of one cell a thread (its
+// 64 frames of 1920 x 1080: 1067 us, against 1382 of one cell a thread (its
 // 274 instructions a cell issued at 65 %; now 187, at 60 % of 42 % of the
 // warps: what is left to hide is the latency of one short launch a
 // generation).  Where rows do not start on 16 bytes, states move in 8-byte
@@ -103,21 +104,8 @@ struct __align__(16) GravTile {
     uint16_t e[XK_GC_WY + 2][XK_GC_P];          // energies, then new energies; column c at c + 2
     float y[XK_GC_WY][XK_GC_P];                 // the gravity every buffer carries; column c at c + 2
     uint8_t sent[XK_GC_WY][XK_GC_PB];           // units sent, by neighbour as xk_gc_bit; column c at c + 2
-    // colours of the inner part's rows: their first 1 to 4 words start on the
-    // word of a 16-byte piece where they start in global memory
-    int4 col[XK_GC_IY][XK_GC_IX / 4 * 3 + 1];
+    int4 col[XK_GC_IY][xk_col_pieces(XK_GC_IX)];    // colours of the inner part (frame.cuh)
 };
-
-// 16 or 4 bytes from global to shared memory; cp.async.wait_all waits for them
-template <int BYTES>
-__device__ __forceinline__ void xk_gc_copy(void *dst, const void *src)
-{
-    const uint32_t to = (uint32_t)__cvta_generic_to_shared(dst);
-    if (BYTES == 16)
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to), "l"(src) : "memory");
-    else
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(to), "l"(src) : "memory");
-}
 
 // The bit of a sent byte that stands for a unit to neighbour j
 __host__ __device__ constexpr uint32_t xk_gc_bit(int j)
@@ -182,30 +170,15 @@ xk_k_gravity(const uint64_t *__restrict__ src, uint64_t *__restrict__ dst, int32
     }
     xk_grid_dep_wait();                 // launched as a dependent of the previous generation
     const bool colours = p.color_kind != XK_COLOR_NONE;
-    // colours move as the 16-byte pieces of a row in order, through shared
-    // memory: three to a lane
     const int width = min(XK_GC_IX, p.W - (x0 + 2));        // cells of a row of the inner part
-    if (colours) {
-        const int64_t words = 3 * (int64_t)p.W * p.H;
+    if (colours)
 #pragma unroll
         for (int r = half; r < XK_GC_IY; r += HALVES) {
             const int gy = y0 + 1 + r;
-            if (gy >= p.H) break;
-            const int64_t first = 3 * ((int64_t)gy * p.W + x0 + 2);
-            const int off = ALIGNED ? 0 : (int)(first & 3);
-            const int *at = col + (first - off);
-            // pieces up to the row's end, whole ones up to the lattice's
-            const int end = off + 3 * width;
-            const int full = ALIGNED ? end : min(end, (int)min(words - (first - off), (int64_t)192) - 3);
-#pragma unroll
-            for (int k = q; k < 48; k += 16)
-                if (4 * k < full) xk_gc_copy<16>(&T.col[r][k], at + 4 * k);
-            if (!ALIGNED && full < end) {       // the lattice's last words
-                const int k = (max(full, 0) + 3 & ~3) + q;
-                if (k < end) xk_gc_copy<4>((int *)T.col[r] + k, at + k);
-            }
+            if (gy < p.H)
+                xk_col_fetch<ALIGNED, XK_GC_IX>(T.col[r], col, 3 * ((int64_t)gy * p.W + x0 + 2), width,
+                                                3 * (int64_t)p.W * p.H, q);
         }
-    }
     uint64_t v[ROWS][2];
 #pragma unroll
     for (int i = 0; i < ROWS; ++i) {
@@ -403,22 +376,10 @@ xk_k_gravity(const uint64_t *__restrict__ src, uint64_t *__restrict__ dst, int32
             }
         }
         if (!colours) continue;
-        const int off = ALIGNED ? 0 : (int)(3 * i & 3);         // the same along a row
-        int *mine = (int *)&T.col[top][0] + off + 12 * min(q, 14);
+        const int64_t first = 3 * ((int64_t)gy * p.W + x0 + 2);
+        int *mine = (int *)T.col[top] + (ALIGNED ? 0 : (int)(first & 3)) + 12 * min(q, 14);
         int c[12];
-        if (ALIGNED) {
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                const int4 o = ((const int4 *)mine)[k];
-                c[4 * k] = o.x;
-                c[4 * k + 1] = o.y;
-                c[4 * k + 2] = o.z;
-                c[4 * k + 3] = o.w;
-            }
-        } else {
-#pragma unroll
-            for (int k = 0; k < 12; ++k) c[k] = mine[k];
-        }
+        xk_col_read<ALIGNED>(mine, c);
         __syncwarp();
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
@@ -427,53 +388,16 @@ xk_k_gravity(const uint64_t *__restrict__ src, uint64_t *__restrict__ dst, int32
             c[3 * k + 1] = xk_fade(gg, c[3 * k + 1], p.fade_in, p.neg_fade_out);
             c[3 * k + 2] = xk_fade(gg, c[3 * k + 2], p.fade_in, p.neg_fade_out);
         }
-        if (in) {
-            if (ALIGNED) {
-#pragma unroll
-                for (int k = 0; k < 3; ++k)
-                    ((int4 *)mine)[k] = make_int4(c[4 * k], c[4 * k + 1], c[4 * k + 2], c[4 * k + 3]);
-            } else {
-#pragma unroll
-                for (int k = 0; k < 12; ++k) mine[k] = c[k];
-            }
-        }
+        if (in) xk_col_write<ALIGNED>(mine, c);
         __syncwarp();
-        if (row_in) {
-            int *at = col + (3 * ((int64_t)gy * p.W + x0 + 2) - off);
-            const int end = off + 3 * width;
-#pragma unroll
-            for (int k = q; k < 48; k += 16) {
-                if (4 * k >= off && 4 * k + 4 <= end) *(int4 *)(at + 4 * k) = T.col[r][k];
-            }
-            if (!ALIGNED) {     // the first and last words: pieces shared with the cells beside
-                const int k = q < 4 ? q : (end & ~3) + q - 4;
-                if (q < 4 ? off > 0 && k >= off && k < end : q < 8 && k >= (off > 0 ? 4 : 0) && k < end)
-                    at[k] = ((const int *)T.col[r])[k];
-            }
-        }
+        if (row_in) xk_col_store<ALIGNED, XK_GC_IX>(T.col[r], col, first, width, q);
         if (!p.frame) continue;
-        int lo = min(c[0], c[1]), hi = max(c[0], c[1]);
-#pragma unroll
-        for (int k = 2; k < 12; k += 2) {
-            lo = __vimin3_s32(lo, c[k], c[k + 1]);
-            hi = __vimax3_s32(hi, c[k], c[k + 1]);
-        }
-        uint32_t px[3][4], b[3];
-#pragma unroll
-        for (int k = 0; k < 12; ++k) px[k % 3][k / 3] = (uint32_t)c[k];
-        xk_pack_px4(px[0], px[1], px[2], b);
-        if (p.frame_smooth > 1 || !xk_px_small(lo) || !xk_px_small(hi))
-#pragma unroll
-            for (int w = 0; w < 3; ++w)
-#pragma unroll 1
-                for (int k = 0; k < 4; ++k) b[w] = b[w] >> 8 | xk_pixel(mine[4 * w + k], p.frame_smooth) << 24;
-        const int first = lane & 16;                     // the row's half warp
+        uint32_t b[3];
+        xk_pixels4(c, mine, p.frame_smooth <= 1 && xk_px_small12(c), p.frame_smooth, b);
+        const int left = lane & 16;                     // the row's half warp
         uint8_t *at = p.frame + 3 * i;
-        xk_store_px4(at, b, lane, first, row_in ? first + width / 4 - 1 : -1);
-        if (!ALIGNED && in && ox + 4 > p.W)              // a row's last one to three cells
-#pragma unroll
-            for (int k = 0; k < 9; ++k)
-                if (ox + k / 3 < p.W) at[k] = (uint8_t)(b[k >> 2] >> (8 * (k & 3)));
+        xk_store_px4(at, b, lane, left, row_in ? left + width / 4 - 1 : -1);
+        if (!ALIGNED && in && ox + 4 > p.W) xk_store_px_rest(at, b, p.W - ox);
     }
 }
 

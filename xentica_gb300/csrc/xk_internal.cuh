@@ -318,8 +318,8 @@ cudaError_t xk_evolife_set_positional(const double *lut54);
 // new colours at zoom 1 with no offset (frame_smooth: its SMOOTH_FACTOR, 0
 // for none)
 cudaError_t xk_evolife_step(const uint64_t *src, uint64_t *dst, int32_t *col, const xk_desc &d,
-                            float mut_thresh, cudaStream_t s, uint8_t *frame = nullptr,
-                            int frame_smooth = 0);
+                            float mut_thresh, const int32_t *col_range, cudaStream_t s,
+                            uint8_t *frame = nullptr, int frame_smooth = 0);
 
 // Life with inherited colour channels (lifecolor.cu): 1 .. max generations,
 // src -> dst, the colours updated, and (frames) each one's zoom-1 frame, one
