@@ -171,3 +171,18 @@ def test_pending_request_can_be_cancelled():
         second.cancel()
         assert second.status() == "cancelled"
         first.result(timeout=120)
+
+
+# 3-D Life-like lattices on clusters of 1 to 16 CTAs (planes fewer than CTAs,
+# slabs of unequal planes, planes of more words than threads, ragged rows,
+# more generations than a round), and one that no cluster holds
+@pytest.mark.parametrize("shape,generations", [
+    ((1, 1, 1), 5), ((1, 9, 33), 12), ((2, 40, 64), 33), ((3, 130, 256), 9), ((13, 64, 64), 1100),
+    ((65, 66, 67), 40), ((37, 256, 256), 12), ((155, 141, 155), 20), ((190, 180, 192), 7), ((256, 200, 256), 5)])
+def test_life3d_shapes(shape, generations):
+    rng = np.random.RandomState(shape[0] + generations)
+    cells = (rng.random_sample(shape) < 0.4).astype(np.uint8)
+    rule = 0b0011000_0010100
+    with serve.Server(1 << 28, quantum=16) as srv:
+        got = srv.submit("life3d", cells, rule, generations).result(timeout=120)
+    assert np.array_equal(got, oracle_result("life3d", cells, rule, generations))

@@ -133,17 +133,7 @@ xk_k_life3d_vn(const uint32_t *__restrict__ src, uint32_t *__restrict__ dst, Lif
     const uint32_t B = __ldg(src + ((int64_t)zb * g.H + y) * g.wpr + j);
     const uint32_t s1 = xk_lop3_xor3(v.L, v.R, U), c1 = xk_maj(v.L, v.R, U);
     const uint32_t s2 = xk_lop3_xor3(Dn, F, B), c2 = xk_maj(Dn, F, B);
-    const uint32_t b0 = s1 ^ s2, c3 = s1 & s2;
-    const uint32_t b1 = xk_lop3_xor3(c1, c2, c3), b2 = xk_maj(c1, c2, c3);
-    uint32_t m[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) m[q] = xk_imux(b0, t.a[q], t.k[q]);
-    uint32_t n[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) n[q] = xk_mux(b1, m[2 * q], m[2 * q + 1]);
-    const uint32_t dead = xk_mux(b2, n[0], n[1]);
-    const uint32_t live = xk_mux(b2, n[2], n[3]);
-    uint32_t out = xk_mux(v.C, dead, live);
+    uint32_t out = xk_life_vn6(t, s1 ^ s2, c1, c2, s1 & s2, v.C);
     if (j == last) out &= g.lastmask;
     dst[idx] = out;
 }

@@ -216,6 +216,21 @@ __device__ __forceinline__ RowVec xk_row_vec(uint32_t c, uint32_t left, uint32_t
     return v;
 }
 
+// The rule bit of 32 cells from six neighbours' count: its bit 0, the three
+// carries at weight 2 (counts 0 .. 6), and the cells
+__device__ __forceinline__ uint32_t xk_life_vn6(const LifeTable &t, uint32_t b0, uint32_t c1, uint32_t c2,
+                                                uint32_t c3, uint32_t cells)
+{
+    const uint32_t b1 = xk_lop3_xor3(c1, c2, c3), b2 = xk_maj(c1, c2, c3);
+    uint32_t m[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) m[q] = xk_imux(b0, t.a[q], t.k[q]);
+    uint32_t n[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) n[q] = xk_mux(b1, m[2 * q], m[2 * q + 1]);
+    return xk_mux(cells, xk_mux(b2, n[0], n[1]), xk_mux(b2, n[2], n[3]));
+}
+
 // neighbour vectors of a torus row: left bit taken from `left` (already the
 // wrapped neighbour word), right bit from `right`; lpre moves the left
 // neighbour's bit to position 31, top / topbit place the right neighbour

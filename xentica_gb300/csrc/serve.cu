@@ -35,7 +35,9 @@
 //   global2d  larger 2-D lattices: packed to 32 cells per word once, one
 //             bit-sliced launch per generation on the request's stream;
 //   life3d    3-D von Neumann Life-like: bit-packed along x like global2d, one
-//             launch per generation;
+//             launch per round on a cluster whose shared memory holds the
+//             lattice (8 x quantum generations a round), else one per
+//             generation;
 //   mass3d    mass transfer: uint32 ping-pong with the per-generation totals
 //             (the fast-only kernel when the submitted total is below 2^30).
 // The other paths run rounds of `quantum` generations.  Full rounds of the
@@ -92,6 +94,7 @@ struct Req {
     int group = -1;            // resident group index
     LifeGeo lg;                // bit-packed rows (3-D: H * D rows)
     Life3Geo g3;
+    Life3ClPlan cl3{0, 0, 0};  // life3d: the cluster that holds it (C 0: none)
     LifeTable lt;
     LifeTable9 lt9;
     int tb_T = 0;              // global2d: generations per temporally blocked launch (0: one per launch)
@@ -442,6 +445,7 @@ static int start_request(xk_server *s, Req *q)
         q->g3.div_wpr = xk_div_magic((uint64_t)q->g3.wpr,
                                      (uint64_t)q->g3.H * (uint64_t)q->g3.D * (uint64_t)q->g3.wpr);
         q->g3.div_h = xk_div_magic((uint64_t)q->g3.H, (uint64_t)q->g3.H * (uint64_t)q->g3.D);
+        if (!xk_life3d_cluster_plan(q->g3, &q->cl3)) q->cl3.C = 0;
         uint32_t *w0 = (uint32_t *)(base + rnd(q->n + 16));
         XK_CUDA(xk_life_pack(base, 1, w0, q->lg, q->stream));
         s->launches++;
@@ -474,6 +478,10 @@ static int enqueue_round(xk_server *s, Req *q, int64_t chunk)
         uint32_t *w[2];
         w[0] = (uint32_t *)(base + rnd(q->n + 16));
         w[1] = (uint32_t *)((uint8_t *)w[0] + rnd((int64_t)q->lg.wpr * q->lg.H * 4));
+        if (q->cl3.C) {
+            XK_CUDA(xk_life_step3d_cluster(w[0], q->g3, q->lt, (int)chunk, q->cl3, q->stream));
+            return XK_OK;
+        }
         if (q->path == PATH_GLOBAL2D && q->tb_T > 1) {
             // temporal blocking: tb_T generations per launch
             for (int64_t g = 0; g < chunk;) {
@@ -508,6 +516,7 @@ static int enqueue_round(xk_server *s, Req *q, int64_t chunk)
 // temporally blocked launch covers up to tb_T generations)
 static int64_t round_flips(const Req *q, int64_t chunk)
 {
+    if (q->cl3.C) return 0;
     if (q->path == PATH_GLOBAL2D && q->tb_T > 1) return (chunk + q->tb_T - 1) / q->tb_T;
     return chunk;
 }
@@ -516,9 +525,9 @@ static int64_t round_flips(const Req *q, int64_t chunk)
 // least two of them left are captured once per parity and replayed
 static int launch_round(xk_server *s, Req *q)
 {
-    const int64_t chunk = std::min(s->quantum, q->r.generations - q->done);
+    const int64_t chunk = std::min(q->cl3.C ? 8 * s->quantum : s->quantum, q->r.generations - q->done);
     const int c0 = q->cur;
-    const bool full = chunk == s->quantum && graphs_enabled();
+    const bool full = chunk == s->quantum && !q->cl3.C && graphs_enabled();
     if (full && !q->graph[c0] && q->r.generations - q->done >= 2 * s->quantum) {
         XK_CUDA(cudaStreamBeginCapture(q->stream, cudaStreamCaptureModeThreadLocal));
         int rc = enqueue_round(s, q, chunk);
@@ -541,7 +550,7 @@ static int launch_round(xk_server *s, Req *q)
         int rc = enqueue_round(s, q, chunk);
         if (rc != XK_OK) return rc;
     }
-    s->launches += round_flips(q, chunk);
+    s->launches += q->cl3.C ? 1 : round_flips(q, chunk);
     XK_CUDA(cudaEventRecord(q->ev, q->stream));
     q->ev_pending = true;
     q->chunk = chunk;

@@ -165,6 +165,14 @@ struct Life3Geo {
 };
 cudaError_t xk_life_step3d_vn(const uint32_t *src, uint32_t *dst, const Life3Geo &g,
                               const LifeTable &t, cudaStream_t s);
+// the same on a cluster of C CTAs that hold the lattice, in place
+// (life3d_cluster.cu); plan returns 0 when it does not fit one
+struct Life3ClPlan {
+    int C, most, smem;         // CTAs, planes of the largest slab, dynamic shared memory
+};
+int xk_life3d_cluster_plan(const Life3Geo &g, Life3ClPlan *out);
+cudaError_t xk_life_step3d_cluster(uint32_t *cells, const Life3Geo &g, const LifeTable &t, int generations,
+                                   const Life3ClPlan &p, cudaStream_t s);
 
 // one lattice (W <= 1024) on a thread-block cluster of C CTAs, R rows each,
 // in place on its bit-packed words (cluster.cu); config returns 0 when no
