@@ -230,6 +230,20 @@ static void quad_shape(QuadParams &p, int &R, bool proj)
     const int64_t sms = xk_sm_count() > 0 ? xk_sm_count() : 1;
     const char *env = getenv("XK_MASS_ZC");
     const int forced = env ? atoi(env) : 0;
+    // the generations of a run ask for the same shape again and again: a
+    // search takes as long as a launch
+    struct Found {
+        int64_t sms;
+        int32_t W, H, D;
+        int forced, zc, R;
+    };
+    static thread_local Found last[2] = {};
+    Found &f = last[proj ? 1 : 0];
+    if (f.R && f.sms == sms && f.W == p.W && f.H == p.H && f.D == p.D && f.forced == forced) {
+        p.zc = f.zc;
+        R = f.R;
+        return;
+    }
     double best = 0;
     p.zc = 1;
     R = 0;
@@ -249,6 +263,7 @@ static void quad_shape(QuadParams &p, int &R, bool proj)
             }
         }
     }
+    f = Found{sms, p.W, p.H, p.D, forced, p.zc, R};
 }
 
 static QuadParams quad_params(const xk_desc &d, int &R, bool proj)

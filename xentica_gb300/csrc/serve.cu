@@ -543,17 +543,24 @@ static int launch_round(xk_server *s, Req *q)
         XK_CUDA(e);
         q->cur = c0;
     }
+    int64_t rounds = 1;
     if (full && q->graph[c0]) {
-        XK_CUDA(cudaGraphLaunch(q->graph[c0], q->stream));
+        // a graph that ends on the buffer it started from runs up to four
+        // times (about 2 ms of a small mass-transfer request, whose 128
+        // generations are followed by up to 40 us until this thread has seen
+        // them end)
+        if (round_flips(q, chunk) % 2 == 0)
+            rounds = std::min<int64_t>(4, (q->r.generations - q->done) / chunk);
+        for (int64_t k = 0; k < rounds; ++k) XK_CUDA(cudaGraphLaunch(q->graph[c0], q->stream));
         q->cur = c0 ^ (int)(round_flips(q, chunk) & 1);
     } else {
         int rc = enqueue_round(s, q, chunk);
         if (rc != XK_OK) return rc;
     }
-    s->launches += q->cl3.C ? 1 : round_flips(q, chunk);
+    s->launches += q->cl3.C ? 1 : rounds * round_flips(q, chunk);
     XK_CUDA(cudaEventRecord(q->ev, q->stream));
     q->ev_pending = true;
-    q->chunk = chunk;
+    q->chunk = rounds * chunk;
     return XK_OK;
 }
 
@@ -621,7 +628,7 @@ static int start_result_copy(xk_server *s, Req *q)
         src = base + (q->cur ? rnd(4 * pn) : 0);
         if (q->r.generations > 0) {
             const unsigned long long *tot = (const unsigned long long *)(base + 2 * rnd(4 * pn));
-            XK_CUDA(cudaMemcpyAsync(hst + rnd(q->n * q->esz), tot + (q->last_chunk - 1), 8,
+            XK_CUDA(cudaMemcpyAsync(hst + rnd(q->n * q->esz), tot + (q->last_chunk - 1) % s->quantum, 8,
                                     cudaMemcpyDeviceToHost, q->stream));
         }
         const int64_t W = q->r.size[0];
