@@ -159,7 +159,7 @@ int xk_step_frames(xk_model *m, int64_t nsteps, int32_t width, int32_t height, i
  * the rows sent by asynchronous remote stores counted in bytes on the
  * receiver's mbarrier (bands of 1 row, or every CTA's bands exactly 2, 4 or
  * 8 rows); TEMPORAL: plan[3] =
- * generations per launch (2..8); DEEP: a cluster that exchanges rows every 8
+ * generations per launch (2..8; 8: as many as pay, 12); DEEP: a cluster that exchanges rows every 8
  * generations, plan[1] = CTAs asked for (1..16), plan[2] = rows per lane group
  * (2, 3, 4 or 6).  xk_model_plan gives kind -1 for models without plans.  A
  * bounded wait of the neighbour, async or deep form that gave up makes the

@@ -63,6 +63,16 @@ def test_depth_matches_oracle(shape, border, depth, monkeypatch):
     assert np.array_equal(got, want)
 
 
+# narrow lattices of heights that take tiles of every height (4 .. 21 rows a
+# warp), and one that ends a row past a tile; 12 + 12 + 7 generations
+@pytest.mark.parametrize("border", ["torus", "static1"])
+@pytest.mark.parametrize("height", [12, 1000, 1217, 3000, 4500, 6000, 8000, 10000, 13000, 17000, 21000])
+def test_tile_heights_match_oracle(height, border, monkeypatch):
+    monkeypatch.setenv("XK_TB", "8")
+    got, want = _run((70, height), border, 31, height)
+    assert np.array_equal(got, want)
+
+
 @pytest.mark.parametrize("shape", [(1500, 700), (4000, 300), (100, 75)])
 def test_tuned_choice_matches_oracle(shape):
     got, want = _run(shape, "torus", 41, 7)

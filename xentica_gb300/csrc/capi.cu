@@ -323,7 +323,7 @@ static int tune_cluster(xk_model *m)
     const size_t bytes = (size_t)m->lg.H * m->lg.wpr * 4;
     uint32_t *scratch = m->bits[1 - m->cur];
     XK_CUDA(cudaMemcpyAsync(scratch, m->bits[m->cur], bytes, cudaMemcpyDeviceToDevice, m->stream));
-    const int G = 32;
+    const int G = 48;
     const int rf = xk_rule_form(m->rule0, m->rule1);
     // device time of `run` (G generations): one untimed run, then the best
     // of three timed ones
@@ -349,7 +349,7 @@ static int tune_cluster(xk_model *m)
         }, &best));
     }
     if (xk_life_tb_supported(m->lg)) {
-        // temporal blocking, 2..8 generations per launch, ping-pong through
+        // temporal blocking, 2 .. 12 generations per launch, ping-pong through
         // a temporary partner of the scratch copy
         uint32_t *tmp = nullptr;
         XK_CUDA(cudaMalloc(&tmp, bytes));
@@ -364,9 +364,10 @@ static int tune_cluster(xk_model *m)
             e = time_it([&]() {
                 uint32_t *a = scratch, *b = tmp;
                 cudaError_t r = cudaSuccess;
-                for (int g = 0; g < G && r == cudaSuccess; g += T) {
+                const int n = xk_life_tb_launch(T);
+                for (int g = 0; g < G && r == cudaSuccess; g += n) {
                     r = T == 1 ? xk_life_step_global(a, b, m->lg, t, m->stream)
-                               : xk_life_step_tb(a, b, m->lg, t9, T, m->stream);
+                               : xk_life_step_tb(a, b, m->lg, t9, n, m->stream);
                     std::swap(a, b);
                 }
                 return r;
@@ -1010,12 +1011,12 @@ static int step_enqueue(xk_model *m, int64_t first, int64_t count, uint8_t *fram
                               m->stream));
         m->cur = 1 - m->cur;
     } else if (m->layout == LAYOUT_BITS2D && colors_free && m->tb_T > 1) {
-        // temporal blocking: launches of tb_T generations, the rest in one
-        // shorter launch; ping-pong between the two word buffers
+        // temporal blocking: launches of tb_T generations (12 for 8), the
+        // rest in one shorter launch; ping-pong between the two word buffers
         const LifeTable9 t9 = xk_life_table9(m->rule0, m->rule1);
         int64_t left = count;
         while (left > 0) {
-            const int T = (int)(left >= m->tb_T ? m->tb_T : left);
+            const int T = (int)std::min<int64_t>(left, xk_life_tb_launch(m->tb_T));
             XK_CUDA(xk_life_step_tb(m->bits[m->cur], m->bits[1 - m->cur], m->lg, t9, T, m->stream));
             m->cur = 1 - m->cur;
             left -= T;

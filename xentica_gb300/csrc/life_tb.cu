@@ -23,16 +23,20 @@
 // incomplete neighbourhoods; their values are never stored.
 //
 // Bound by the logic pipe (63 %; 39 instructions a word, of which a rule read
-// from a table is 18).  4096 x 4096, such a rule, 1000 generations and the
-// read after them: 1 803 us, against 2 536 us with the tile in shared memory
-// (every word of every generation loaded, stored and waited for).
+// from a table is 18) and by about 3 us a launch (its start, the tile's loads
+// and stores).  4096 x 4096, such a rule, 960 generations: 1 295 us with 12
+// generations a launch and tiles of 21 rows a warp (144 of the 152 SMs hold
+// one; 1 310 with 16 generations), 1 414 with 8, 1 605 with 8 on tiles of 12
+// rows a warp (two on most SMs, one on the others); twice that with the tile
+// in shared memory (every word of every generation loaded, stored and waited
+// for).
 //
 // Requires W >= 64 (a 32-cell window wraps at most once).
 #include <string.h>
 
 #include "life_word.cuh"
 
-#define XK_TB_MAXT 8
+#define XK_TB_MAXT XK_TB_DEEPEST
 #define XK_TB_WARPS 8
 
 struct TbParams {
@@ -159,11 +163,14 @@ cudaError_t xk_life_step_tb(const uint32_t *src, uint32_t *dst, const LifeGeo &g
     // Rows a warp: the height whose tiles, dealt to the SMs, leave the
     // fewest rows on the fullest one (ties: the taller, less halo).
     const int64_t gx = (g.W + 30 * 32 - 1) / (30 * 32), sms = xk_sm_count() > 0 ? xk_sm_count() : 1;
-    static const int heights[] = {16, 12, 8, 4};
+    // Against heights of 16, 12, 8 and 4 alone, 12 generations of lattices
+    // with sides up to 4000 and at least 2^20 cells take 22 % fewer rows.
+    static const int heights[] = {21, 17, 14, 12, 10, 8, 7, 6, 5, 4};
     int B = 0;
     int64_t best = 0;
     for (int b : heights) {
         const int th = XK_TB_WARPS * b - 2 * T;
+        if (th <= 0) continue;
         const int64_t tiles = gx * ((g.H + th - 1) / th), rows = (tiles + sms - 1) / sms * XK_TB_WARPS * b;
         if (!B || rows < best) {
             B = b;
@@ -179,7 +186,18 @@ cudaError_t xk_life_step_tb(const uint32_t *src, uint32_t *dst, const LifeGeo &g
     // B3/S23 runs the instantiation with the rule compiled in
     const LifeTable9 table = xk_life_table9(8u, 12u);
     const bool conway = memcmp(&t, &table, sizeof(t)) == 0, torus = g.torus != 0;
-    const TbKernel k = B == 16 ? tb_kernel<16>(torus, conway) : B == 12 ? tb_kernel<12>(torus, conway)
-                       : B == 8 ? tb_kernel<8>(torus, conway) : tb_kernel<4>(torus, conway);
+    TbKernel k = nullptr;
+    switch (B) {
+    case 4: k = tb_kernel<4>(torus, conway); break;
+    case 5: k = tb_kernel<5>(torus, conway); break;
+    case 6: k = tb_kernel<6>(torus, conway); break;
+    case 7: k = tb_kernel<7>(torus, conway); break;
+    case 8: k = tb_kernel<8>(torus, conway); break;
+    case 10: k = tb_kernel<10>(torus, conway); break;
+    case 12: k = tb_kernel<12>(torus, conway); break;
+    case 14: k = tb_kernel<14>(torus, conway); break;
+    case 17: k = tb_kernel<17>(torus, conway); break;
+    default: k = tb_kernel<21>(torus, conway); break;
+    }
     return xk_launch_pdl(k, grid, dim3(32 * XK_TB_WARPS), 0, s, src, dst, p, t);
 }

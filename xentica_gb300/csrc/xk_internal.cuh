@@ -217,9 +217,16 @@ int xk_life_deep_config(const LifeGeo &g, int C, int B, DeepPlan *out);
 cudaError_t xk_life_step_deep(uint32_t *bits, const LifeGeo &g, uint32_t rule0, uint32_t rule1, int generations,
                               const DeepPlan &p, unsigned int *gave_up, cudaStream_t s);
 
-// T (1..8) generations per launch of a 2-D lattice of any size (W >= 64),
-// tiles with a T-generation halo in shared memory, src -> dst (life_tb.cu)
+// T (1 .. XK_TB_DEEPEST) generations per launch of a 2-D lattice of any size
+// (W >= 64), tiles with a T-generation halo in registers, src -> dst
+// (life_tb.cu)
+#define XK_TB_DEEPEST 12
 int xk_life_tb_supported(const LifeGeo &g);
+// generations of a launch of a plan of this depth (2 .. 8): a depth of 8 asks
+// for as many as pay.  960 generations take 1 295 us of 12 a launch and 1 414
+// of 8 at 4096 x 4096, 454 and 473 at 1100 x 1100, 554 and 574 at 2000 x 1500;
+// 16 are up to 8 % slower at some sizes, 3 % faster at others.
+inline int xk_life_tb_launch(int depth) { return depth == 8 ? XK_TB_DEEPEST : depth; }
 cudaError_t xk_life_step_tb(const uint32_t *src, uint32_t *dst, const LifeGeo &g, const LifeTable9 &t,
                             int T, cudaStream_t s);
 
