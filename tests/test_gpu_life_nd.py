@@ -47,3 +47,26 @@ def test_against_oracle(kind, size, border):
     O.life_run(topo, fld, col, 4, born=rule, sustain=rule >> 9)
     assert np.array_equal(model.gpu.arrays.cells.get()[:model.cells_num], fld[:topo.cells])
     assert np.array_equal(model.gpu.arrays.colors.get(), col)
+
+
+# 3-D von Neumann lattices on clusters of 1 to 16 CTAs (fewer planes than
+# CTAs, slabs of unequal planes, planes of more words than threads), and one
+# that no cluster holds
+@pytest.mark.parametrize("size", [(1, 1, 1), (33, 9, 1), (64, 40, 2), (256, 130, 3), (64, 64, 13), (67, 66, 65),
+                                  (256, 256, 20), (155, 141, 55), (192, 180, 190), (256, 200, 256)])
+@pytest.mark.parametrize("border", [None, 0, 1])
+def test_faces_against_oracle(size, border):
+    rng = np.random.RandomState(sum(size))
+    rule = 4 | 12 << 9 if border == 0 else int(rng.randint(0, 2 ** 31 - 1))
+    exp = type("E", (GOLExperiment2, ), {"size": size, "rule": rule})
+    model = _model("von_neumann", 3, border)(exp)
+    n = model.cells_num
+    cells = (rng.random_sample(n) < 0.3).astype(np.uint8)
+    model.gpu.load(cells, np.zeros(3 * n, dtype=np.int32))
+    topo = O.Topology(size, "von_neumann", border)
+    fld = topo.field(cells, np.uint8)
+    col = np.zeros(topo.cells * 3, dtype=np.int32)
+    for k in (1, 11, 2):
+        model.gpu.step(k)
+        O.life_run(topo, fld, col, k, born=rule, sustain=rule >> 9)
+        assert np.array_equal(model.gpu.arrays.cells.get()[:n], fld[:n]), k

@@ -161,6 +161,8 @@ struct xk_model {
     LifeGeo lg;
     NdGeo ng;
     BitsNdGeo bg;                // LAYOUT_BITSND (lg: its packing, n / W rows)
+    Life3Geo g3;                 // of it, 3-D von Neumann (bg.faces3d): geometry and the
+    Life3ClPlan cl3{0, 0, 0};    // cluster that holds the lattice (C 0: none)
     uint32_t *bits[2] = {nullptr, nullptr};
     uint8_t *bytes[2] = {nullptr, nullptr};
     uint64_t *cells64[2] = {nullptr, nullptr};  // EvoLife, GraviCowboys: reference layout, ping-pong
@@ -631,6 +633,10 @@ extern "C" int xk_model_create(const xk_desc *desc, xk_model **out)
             if (d.family == XK_FAMILY_LIFE && xk_bits_nd_geo(m->ng, &m->bg)) {
                 m->layout = LAYOUT_BITSND;
                 m->lg = xk_life_geo(d.size[0], n / d.size[0], d.torus, border_state);
+                if (m->bg.faces3d) {
+                    m->g3 = xk_life3_geo(d.size[0], d.size[1], d.size[2], d.torus, border_state);
+                    if (!xk_life3d_cluster_plan(m->g3, true, &m->cl3)) m->cl3.C = 0;
+                }
                 const size_t words = (size_t)m->bg.words;
                 XK_TRY(cudaMalloc(&m->bits[0], (words + 4) * 4));
                 XK_TRY(cudaMalloc(&m->bits[1], (words + 4) * 4));
@@ -994,6 +1000,12 @@ static int step_enqueue(xk_model *m, int64_t first, int64_t count, uint8_t *fram
         for (int64_t left = count; left > 0; left -= 4096)
             XK_CUDA(xk_life_step_deep(m->bits[m->cur], m->lg, m->rule0, m->rule1,
                                       (int)std::min<int64_t>(left, 4096), m->deep, m->gave_up, m->stream));
+    } else if (m->layout == LAYOUT_BITSND && colors_free && m->cl3.C && count > 1) {
+        // a 3-D von Neumann lattice on a cluster, in place
+        const LifeTable t = xk_life_table(m->rule0, m->rule1);
+        for (int64_t left = count; left > 0; left -= 4096)
+            XK_CUDA(xk_life_step3d_cluster(m->bits[m->cur], m->g3, t, (int)std::min<int64_t>(left, 4096), m->cl3,
+                                           m->stream));
     } else if (m->layout == LAYOUT_BITS2D && colors_free && m->cl_C) {
         // whole lattice in the shared memory of a cluster; long runs are cut
         // into launches of at most 4096 generations
@@ -1047,7 +1059,9 @@ static int step_enqueue(xk_model *m, int64_t first, int64_t count, uint8_t *fram
                     m->cur = 1 - m->cur;
                 }
             } else {
-                if (m->layout == LAYOUT_BITSND)
+                if (m->layout == LAYOUT_BITSND && m->bg.faces3d)
+                    XK_CUDA(xk_life_step3d_vn(m->bits[m->cur], m->bits[1 - m->cur], m->g3, t, m->stream));
+                else if (m->layout == LAYOUT_BITSND)
                     XK_CUDA(xk_life_step_bits_nd(m->bits[m->cur], m->bits[1 - m->cur], m->bg, m->rule0,
                                                  m->rule1, m->stream));
                 else if (m->d.family == XK_FAMILY_SHIFT)

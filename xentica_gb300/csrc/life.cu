@@ -99,8 +99,8 @@ cudaError_t xk_life_step_global(const uint32_t *src, uint32_t *dst, const LifeGe
 }
 
 // ---------------------------------------------------------------------------
-// 3-D von Neumann Life-like on a torus (the serving loop's 3-D requests),
-// bit-packed along x: row (y, z) is row z * H + y of the 2-D packing, so the
+// 3-D von Neumann Life-like (the serving loop's 3-D requests, models that no
+// cluster holds), bit-packed along x: row (y, z) is row z * H + y of the 2-D packing, so the
 // pack/unpack kernels above serve unchanged with H * D rows.  One thread per
 // word: the x neighbours come from the row's own words (torus wrap as in 2-D),
 // y and z neighbours are the same word of four other rows.  Six one-bit
@@ -108,6 +108,7 @@ cudaError_t xk_life_step_global(const uint32_t *src, uint32_t *dst, const LifeGe
 // carries; the count and the cell's state select the rule bit through the
 // same multiplexer tree as in 2-D (counts 0..6).
 
+template <bool TORUS>
 __global__ void __launch_bounds__(256)
 xk_k_life3d_vn(const uint32_t *__restrict__ src, uint32_t *__restrict__ dst, Life3Geo g,
                LifeTable t)
@@ -123,19 +124,43 @@ xk_k_life3d_vn(const uint32_t *__restrict__ src, uint32_t *__restrict__ dst, Lif
     const int lshift = j > 0 ? 31 : g.rlast - 1;
     const int top = j == last ? g.rlast - 1 : 31;
     const uint32_t *row = src + r * g.wpr;
-    const RowVec v = xk_row_vec(__ldg(row + j), __ldg(row + jl), __ldg(row + jr), lshift, top, 0u,
-                                0u, 0, 0);
+    const uint32_t edge = TORUS ? 0u : g.bfill & 1u;
+    const RowVec v = xk_row_vec(__ldg(row + j), __ldg(row + jl), __ldg(row + jr), lshift, top, edge, edge,
+                                !TORUS && j == 0, !TORUS && j == last);
     const int yu = y > 0 ? y - 1 : g.H - 1, yd = y + 1 < g.H ? y + 1 : 0;
     const int zf = z > 0 ? z - 1 : g.D - 1, zb = z + 1 < g.D ? z + 1 : 0;
-    const uint32_t U = __ldg(src + ((int64_t)z * g.H + yu) * g.wpr + j);
-    const uint32_t Dn = __ldg(src + ((int64_t)z * g.H + yd) * g.wpr + j);
-    const uint32_t F = __ldg(src + ((int64_t)zf * g.H + y) * g.wpr + j);
-    const uint32_t B = __ldg(src + ((int64_t)zb * g.H + y) * g.wpr + j);
+    uint32_t U = __ldg(src + ((int64_t)z * g.H + yu) * g.wpr + j);
+    uint32_t Dn = __ldg(src + ((int64_t)z * g.H + yd) * g.wpr + j);
+    uint32_t F = __ldg(src + ((int64_t)zf * g.H + y) * g.wpr + j);
+    uint32_t B = __ldg(src + ((int64_t)zb * g.H + y) * g.wpr + j);
+    if (!TORUS) {
+        U = y > 0 ? U : g.bfill;
+        Dn = y + 1 < g.H ? Dn : g.bfill;
+        F = z > 0 ? F : g.bfill;
+        B = z + 1 < g.D ? B : g.bfill;
+    }
     const uint32_t s1 = xk_lop3_xor3(v.L, v.R, U), c1 = xk_maj(v.L, v.R, U);
     const uint32_t s2 = xk_lop3_xor3(Dn, F, B), c2 = xk_maj(Dn, F, B);
     uint32_t out = xk_life_vn6(t, s1 ^ s2, c1, c2, s1 & s2, v.C);
     if (j == last) out &= g.lastmask;
     dst[idx] = out;
+}
+
+Life3Geo xk_life3_geo(int64_t W, int64_t H, int64_t D, int torus, int border_state)
+{
+    const LifeGeo lg = xk_life_geo(W, H * D, torus, border_state);
+    Life3Geo g;
+    g.W = (int32_t)W;
+    g.H = (int32_t)H;
+    g.D = (int32_t)D;
+    g.wpr = lg.wpr;
+    g.rlast = lg.rlast;
+    g.lastmask = lg.lastmask;
+    g.div_wpr = xk_div_magic((uint64_t)g.wpr, (uint64_t)H * (uint64_t)D * (uint64_t)g.wpr);
+    g.div_h = xk_div_magic((uint64_t)H, (uint64_t)H * (uint64_t)D);
+    g.torus = lg.torus;
+    g.bfill = lg.bfill;
+    return g;
 }
 
 cudaError_t xk_life_step3d_vn(const uint32_t *src, uint32_t *dst, const Life3Geo &g,
@@ -145,7 +170,8 @@ cudaError_t xk_life_step3d_vn(const uint32_t *src, uint32_t *dst, const Life3Geo
     if (total > 0xFFFFFFFFll) return cudaErrorInvalidValue;   // 32-bit word indices
     const int threads = 256;
     const int64_t blocks = (total + threads - 1) / threads;
-    return xk_launch_pdl(xk_k_life3d_vn, dim3((unsigned)blocks), dim3(threads), 0, s, src, dst, g, t);
+    return g.torus ? xk_launch_pdl(xk_k_life3d_vn<true>, dim3((unsigned)blocks), dim3(threads), 0, s, src, dst, g, t)
+                   : xk_launch_pdl(xk_k_life3d_vn<false>, dim3((unsigned)blocks), dim3(threads), 0, s, src, dst, g, t);
 }
 
 // ---------------------------------------------------------------------------

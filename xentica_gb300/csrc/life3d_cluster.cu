@@ -1,6 +1,5 @@
-// A 3-D von Neumann Life-like lattice on a torus, bit-packed along x, in the
-// shared memory of a thread-block cluster for all generations of a launch
-// (the serving loop's 3-D requests).
+// A 3-D von Neumann Life-like lattice, bit-packed along x, in the shared memory
+// of a thread-block cluster for all generations of a launch.
 //
 // The planes are cut into slabs, one a CTA.  A CTA keeps its slab twice
 // (ping-pong) with the plane below and above it: a generation reads one copy,
@@ -10,11 +9,14 @@
 // and walks up it with the words below, at and above in registers: a word
 // costs one new load along z and four beside it.
 //
-// Many requests run at once, and a generation of one is a launch of 1 to 3 us
-// of work elsewhere (xk_k_life3d_vn): the chip starts less than one launch a
-// microsecond, so 9 such requests among 32 mixed ones spent most of their time
-// between launches.  Here a request takes a few SMs and one launch for many
-// generations.  XXXX
+// Served lattices: many requests run at once, and a generation of one is a
+// launch of its own elsewhere (xk_k_life3d_vn); 9 such requests made 8500 of
+// the 15 700 launches of 32 mixed ones.  Here a request takes a few SMs and one
+// launch for many generations: the 32 took 26.2 ms before and 23.6 with it.
+// A lattice alone: bound by the cluster barrier, 1.4 to 1.5 us a generation up
+// to 32 768 words (64^3 1.51, 160 x 50 x 40 1.38; one launch a generation, whose
+// launches overlap, 1.63 and 1.89; 4.5 with the kernel of any neighbourhood);
+// beyond, by the words its 16 SMs work through: 128^3 2.2 against 1.7.
 #include <string.h>
 
 #include <algorithm>
@@ -29,6 +31,7 @@ __device__ __forceinline__ void xk_l3_store_remote(uint32_t addr, uint32_t v)
     asm volatile("st.shared::cluster.u32 [%0], %1;" : : "r"(addr), "r"(v) : "memory");
 }
 
+template <bool TORUS>
 __global__ void __launch_bounds__(XK_L3_THREADS, 1)
 xk_k_life3d_cluster(uint32_t *__restrict__ cells, Life3Geo g, const __grid_constant__ LifeTable t, int C,
                     int most, int gens)
@@ -45,9 +48,18 @@ xk_k_life3d_cluster(uint32_t *__restrict__ cells, Life3Geo g, const __grid_const
     const uint32_t to_next = xk_cl_mapa(own, next);
     for (int w = tid; w < n * P; w += XK_L3_THREADS) sm[P + w] = cells[(int64_t)z0 * P + w];
     for (int w = tid; w < P; w += XK_L3_THREADS) {
-        sm[w] = cells[(int64_t)(z0 > 0 ? z0 - 1 : g.D - 1) * P + w];
-        sm[(n + 1) * P + w] = cells[(int64_t)(z1 < g.D ? z1 : 0) * P + w];
+        uint32_t below = cells[(int64_t)(z0 > 0 ? z0 - 1 : g.D - 1) * P + w];
+        uint32_t above = cells[(int64_t)(z1 < g.D ? z1 : 0) * P + w];
+        if (!TORUS) {
+            // a border's planes are in both copies: nobody sends them
+            if (z0 == 0) sm[buf + w] = below = g.bfill;
+            if (z1 == g.D) sm[buf + (n + 1) * P + w] = above = g.bfill;
+        }
+        sm[w] = below;
+        sm[(n + 1) * P + w] = above;
     }
+    const bool send_prev = TORUS || rank > 0, send_next = TORUS || rank + 1 < C;
+    const uint32_t edge = TORUS ? 0u : g.bfill & 1u;
     // a plane of up to half the threads' columns is walked in several runs
     const int runs = max(1, min(n, XK_L3_THREADS / P));
     const int run = P < XK_L3_THREADS ? tid / P : 0;
@@ -69,14 +81,20 @@ xk_k_life3d_cluster(uint32_t *__restrict__ cells, Life3Geo g, const __grid_const
                 uint32_t below = s[-P], at = s[0];
 #pragma unroll 2
                 for (int z = za; z < zb; ++z) {
-                    const uint32_t above = s[P], U = s[u], Dn = s[d];
-                    const RowVec v = xk_row_vec(at, s[l], s[r], lshift, top, 0u, 0u, 0, 0);
+                    const uint32_t above = s[P];
+                    uint32_t U = s[u], Dn = s[d];
+                    if (!TORUS) {
+                        U = y > 0 ? U : g.bfill;
+                        Dn = y + 1 < g.H ? Dn : g.bfill;
+                    }
+                    const RowVec v = xk_row_vec(at, s[l], s[r], lshift, top, edge, edge, !TORUS && j == 0,
+                                                !TORUS && j == last);
                     const uint32_t s1 = xk_lop3_xor3(v.L, v.R, U), c1 = xk_maj(v.L, v.R, U);
                     const uint32_t s2 = xk_lop3_xor3(Dn, below, above), c2 = xk_maj(Dn, below, above);
                     const uint32_t out = xk_life_vn6(t, s1 ^ s2, c1, c2, s1 & s2, at) & mask;
                     *o = out;
-                    if (z == 1) xk_l3_store_remote(to_prev + 4u * (uint32_t)(into + col), out);
-                    if (z == n) xk_l3_store_remote(to_next + 4u * (uint32_t)(into + col), out);
+                    if (z == 1 && send_prev) xk_l3_store_remote(to_prev + 4u * (uint32_t)(into + col), out);
+                    if (z == n && send_next) xk_l3_store_remote(to_next + 4u * (uint32_t)(into + col), out);
                     below = at;
                     at = above;
                     s += P;
@@ -105,33 +123,40 @@ static void l3_cfg(cudaLaunchConfig_t &cfg, cudaLaunchAttribute &attr, const Lif
     cfg.numAttrs = 1;
 }
 
-static cudaError_t l3_attrs(int smem)
+typedef void (*L3Kernel)(uint32_t *, Life3Geo, LifeTable, int, int, int);
+
+static L3Kernel l3_kernel(const Life3Geo &g) { return g.torus ? xk_k_life3d_cluster<true> : xk_k_life3d_cluster<false>; }
+
+static cudaError_t l3_attrs(const Life3Geo &g, int smem)
 {
-    const void *k = (const void *)xk_k_life3d_cluster;
+    const void *k = (const void *)l3_kernel(g);
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     return e != cudaSuccess || smem <= 48 * 1024 ? e : xk_smem_attr_at_least(k, smem);
 }
 
-int xk_life3d_cluster_plan(const Life3Geo &g, Life3ClPlan *out)
+int xk_life3d_cluster_plan(const Life3Geo &g, bool alone, Life3ClPlan *out)
 {
     const int64_t P = (int64_t)g.H * g.wpr, words = P * g.D;
     if (words > (int64_t)16 * xk_max_smem_optin()) return 0;
     // CTAs of about 2048 words (a microsecond a generation, half of it the
-    // barrier), at most 8 of them, more only where they hold the lattice
+    // barrier), at most 8 of them beside other work, more only where they
+    // hold the lattice
+    const int enough = alone ? 16 : 8;
+    if (alone && words > 2048 * 16) return 0;       // one launch a generation is faster
     for (int C = 1; C <= 16; C *= 2) {
         if (C > g.D) return 0;
         Life3ClPlan p;
         p.C = C;
         p.most = (g.D + C - 1) / C;
         const int64_t smem = 8 * (int64_t)(p.most + 2) * P;
-        if (smem > xk_max_smem_optin() || (C < 8 && 2 * C <= g.D && words > 2048 * (int64_t)C)) continue;
+        if (smem > xk_max_smem_optin() || (C < enough && 2 * C <= g.D && words > 2048 * (int64_t)C)) continue;
         p.smem = (int)smem;
         cudaLaunchConfig_t cfg;
         cudaLaunchAttribute attr;
         l3_cfg(cfg, attr, p, 0);
         int active = 0;
-        if (l3_attrs(p.smem) != cudaSuccess ||
-            cudaOccupancyMaxActiveClusters(&active, (const void *)xk_k_life3d_cluster, &cfg) != cudaSuccess ||
+        if (l3_attrs(g, p.smem) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&active, (const void *)l3_kernel(g), &cfg) != cudaSuccess ||
             active < 1) {
             cudaGetLastError();
             return 0;
@@ -145,10 +170,10 @@ int xk_life3d_cluster_plan(const Life3Geo &g, Life3ClPlan *out)
 cudaError_t xk_life_step3d_cluster(uint32_t *cells, const Life3Geo &g, const LifeTable &t, int generations,
                                    const Life3ClPlan &p, cudaStream_t s)
 {
-    cudaError_t e = l3_attrs(p.smem);
+    cudaError_t e = l3_attrs(g, p.smem);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr;
     l3_cfg(cfg, attr, p, s);
-    return cudaLaunchKernelEx(&cfg, xk_k_life3d_cluster, cells, g, t, p.C, p.most, generations);
+    return cudaLaunchKernelEx(&cfg, l3_kernel(g), cells, g, t, p.C, p.most, generations);
 }

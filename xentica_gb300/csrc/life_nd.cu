@@ -10,6 +10,9 @@
 // and the cells select the rule bit through a multiplexer tree over
 // warp-uniform masks, as in life_word.cuh.
 //
+// The six faces of a 3-D lattice have kernels of their own (life.cu,
+// life3d_cluster.cu): 100 generations of 128^3 450 -> 169 us.
+//
 // Bound by the launch, not by the arithmetic: a 128^3 lattice is 65 536 words
 // of about 210 instructions (0.35 us of issue on 152 SMs) and 262 KB that stay
 // in L2.  100 generations of 128^3 Moore and the read after them: 432 us,
@@ -239,6 +242,10 @@ int xk_bits_nd_geo(const NdGeo &nd, BitsNdGeo *out)
         g.delta[at][0] = (int8_t)(g.delta[at][0] | bit);
     }
     g.nbr = nd.nbr;
+    // the six faces, in any order
+    g.faces3d = nd.ndim == 3 && nd.nbr == 6;
+    for (int k = 0; k < nd.nbr && g.faces3d; ++k)
+        g.faces3d = abs(nd.delta[k][0]) + abs(nd.delta[k][1]) + abs(nd.delta[k][2]) == 1;
     // 26 of the 27 offsets, (1, 1, 1) the one left out
     g.moore3d = 0;
     if (nd.ndim == 3 && nd.nbr == 26) {

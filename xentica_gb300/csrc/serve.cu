@@ -436,16 +436,8 @@ static int start_request(xk_server *s, Req *q)
         q->rule1 = life3d_rule1(r.rule);
         q->lg = xk_life_geo(r.size[0], r.size[1] * r.size[2], 1, 0);
         q->lt = xk_life_table(q->rule0, q->rule1);
-        q->g3.W = (int32_t)r.size[0];
-        q->g3.H = (int32_t)r.size[1];
-        q->g3.D = (int32_t)r.size[2];
-        q->g3.wpr = q->lg.wpr;
-        q->g3.rlast = q->lg.rlast;
-        q->g3.lastmask = q->lg.lastmask;
-        q->g3.div_wpr = xk_div_magic((uint64_t)q->g3.wpr,
-                                     (uint64_t)q->g3.H * (uint64_t)q->g3.D * (uint64_t)q->g3.wpr);
-        q->g3.div_h = xk_div_magic((uint64_t)q->g3.H, (uint64_t)q->g3.H * (uint64_t)q->g3.D);
-        if (!xk_life3d_cluster_plan(q->g3, &q->cl3)) q->cl3.C = 0;
+        q->g3 = xk_life3_geo(r.size[0], r.size[1], r.size[2], 1, 0);
+        if (!xk_life3d_cluster_plan(q->g3, false, &q->cl3)) q->cl3.C = 0;
         uint32_t *w0 = (uint32_t *)(base + rnd(q->n + 16));
         XK_CUDA(xk_life_pack(base, 1, w0, q->lg, q->stream));
         s->launches++;

@@ -156,13 +156,17 @@ cudaError_t xk_life_color_step(const uint32_t *bits, int32_t *col, const LifeGeo
                                const int32_t *lut6, int fade_in, int fade_out, int smooth,
                                int plain, cudaStream_t s);
 
-// 3-D von Neumann Life-like on a torus, bit-packed along x; row (y, z) is row
-// z * H + y (pack/unpack with xk_life_geo(W, H * D, 1, 0))
+// 3-D von Neumann Life-like, bit-packed along x; row (y, z) is row z * H + y
+// (pack/unpack with xk_life_geo(W, H * D, torus, border state))
 struct Life3Geo {
     int32_t W, H, D, wpr, rlast;
     uint32_t lastmask;
     uint32_t div_wpr, div_h;   // xk_div_magic(wpr, H * D * wpr), xk_div_magic(H, H * D)
+    int32_t torus;
+    uint32_t bfill;            // static border: its state in every bit
 };
+// (div_h only for lattices of fewer than 2^32 words, which the kernels take)
+Life3Geo xk_life3_geo(int64_t W, int64_t H, int64_t D, int torus, int border_state);
 cudaError_t xk_life_step3d_vn(const uint32_t *src, uint32_t *dst, const Life3Geo &g,
                               const LifeTable &t, cudaStream_t s);
 // the same on a cluster of C CTAs that hold the lattice, in place
@@ -170,7 +174,7 @@ cudaError_t xk_life_step3d_vn(const uint32_t *src, uint32_t *dst, const Life3Geo
 struct Life3ClPlan {
     int C, most, smem;         // CTAs, planes of the largest slab, dynamic shared memory
 };
-int xk_life3d_cluster_plan(const Life3Geo &g, Life3ClPlan *out);
+int xk_life3d_cluster_plan(const Life3Geo &g, bool alone, Life3ClPlan *out);
 cudaError_t xk_life_step3d_cluster(uint32_t *cells, const Life3Geo &g, const LifeTable &t, int generations,
                                    const Life3ClPlan &p, cudaStream_t s);
 
@@ -241,7 +245,7 @@ struct NdGeo {
 // grouped by row (delta[k][1..]; delta[k][0]: bit 0 the left, 1 the middle, 2
 // the right cell of the row)
 struct BitsNdGeo {
-    int32_t ndim, nbr, groups, torus, moore3d;
+    int32_t ndim, nbr, groups, torus, moore3d, faces3d;
     int32_t size[XK_MAXDIM];
     int8_t delta[XK_MAXNBR][XK_MAXDIM];
     int32_t wpr, rlast;
