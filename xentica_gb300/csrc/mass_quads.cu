@@ -24,8 +24,9 @@
 // (tensor copies into a shared ring, a barrier a plane, 163 instructions a warp
 // and plane): 64^3 2.4 (3.4), 128^3 3.7 (5.5), 129 x 118 x 72 3.3 (5.5), 171 x
 // 205 x 215 10.6 (16.9), 256^3 21.2 (24.5; 25.2 with every generation marching
-// the same way); with a frame each 128^3 5.0 (7.5), 256^3 27.0
-// (29.9).
+// the same way); with a frame each 128^3 5.0 (7.5), 256^3 26.5
+// (29.9; 27.0 with the column sums in registers and the frame before the first
+// planes' loads).
 #include <string.h>
 
 #include "xk_internal.cuh"
@@ -49,6 +50,11 @@ __device__ __forceinline__ uint4 pick(bool a, const uint4 &x, const uint4 &y)
 }
 
 __device__ __forceinline__ uint32_t colour(uint32_t m) { return min(m * 32u, 255u); }
+
+__device__ __forceinline__ void add_shared(uint32_t at, uint32_t v)
+{
+    asm volatile("red.shared.add.u32 [%0], %1;" : : "r"(at), "r"(v) : "memory");
+}
 
 }  // namespace
 
@@ -80,9 +86,27 @@ xk_k_mass_quads(const uint32_t *__restrict__ src, uint32_t *__restrict__ dst, un
     const bool halo = lane == 0 ? !first : lane == 31 && !last;
     const int halo_at = lane == 0 ? -1 : 4;
     xk_grid_dep_wait();       // launched as a dependent of the previous generation
+    // q of the plane before, cells and q of this one, its rows above and
+    // below and halo cells as loaded
+    uint4 qp[R], m[R], q[R], mu, md;
+    uint32_t mh[R];
+    {
+        const int z = p.back ? z1 - 1 : z0;
+        const uint4 *a = cell + (int64_t)z * plane;
+#pragma unroll
+        for (int r = 0; r < R; ++r) m[r] = __ldg(a + r * pitch);
+        mu = __ldg(a + up);
+        md = __ldg(a + down);
+#pragma unroll
+        for (int r = 0; r < R; ++r) mh[r] = halo ? __ldg((const uint32_t *)(a + r * pitch) + halo_at) : 0u;
+        const uint4 *b = cell + (int64_t)(p.back ? min(z + 1, p.D - 1) : max(z - 1, 0)) * plane;
+#pragma unroll
+        for (int r = 0; r < R; ++r) qp[r] = __ldg(b + r * pitch);
+    }
     if (PROJ && frame_prev) {
         // the previous generation's frame, four pixels a thread over the
         // whole grid, and its sums zeroed for the generation after this one
+        // (here, while the first planes are on their way)
         const uint32_t quads = pitch * (uint32_t)p.H, threads = gridDim.x * gridDim.y * 128u;
         for (uint32_t i = blockIdx.y * gridDim.x * 128u + t; i < quads; i += threads) {
             const uint4 c = ((const uint4 *)proj_prev)[i];
@@ -105,32 +129,19 @@ xk_k_mass_quads(const uint32_t *__restrict__ src, uint32_t *__restrict__ dst, un
             }
         }
     }
-    // q of the plane before, cells and q of this one, its rows above and
-    // below and halo cells as loaded
-    uint4 qp[R], m[R], q[R], mu, md;
-    uint32_t mh[R];
-    {
-        const int z = p.back ? z1 - 1 : z0;
-        const uint4 *a = cell + (int64_t)z * plane;
 #pragma unroll
-        for (int r = 0; r < R; ++r) m[r] = __ldg(a + r * pitch);
-        mu = __ldg(a + up);
-        md = __ldg(a + down);
-#pragma unroll
-        for (int r = 0; r < R; ++r) mh[r] = halo ? __ldg((const uint32_t *)(a + r * pitch) + halo_at) : 0u;
-        const uint4 *b = cell + (int64_t)(p.back ? min(z + 1, p.D - 1) : max(z - 1, 0)) * plane;
-#pragma unroll
-        for (int r = 0; r < R; ++r) qp[r] = __ldg(b + r * pitch);
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            qp[r] = q7(qp[r]);
-            q[r] = q7(m[r]);
-        }
+    for (int r = 0; r < R; ++r) {
+        qp[r] = q7(qp[r]);
+        q[r] = q7(m[r]);
     }
     uint32_t sum = 0;                       // below 2^30: the whole lattice's total is
-    uint32_t cs[R][2];
+    // column sums, two 16-bit ones a word, in this thread's own words of
+    // shared memory: added to without waiting, and no registers of the loop
+    __shared__ uint32_t column[PROJ ? 2 * R : 1][128];
+    const uint32_t mine = (uint32_t)__cvta_generic_to_shared(&column[0][threadIdx.x]);
+    if (PROJ)
 #pragma unroll
-    for (int r = 0; r < R; ++r) cs[r][0] = cs[r][1] = 0u;
+        for (int r = 0; r < 2 * R; ++r) column[PROJ ? r : 0][threadIdx.x] = 0u;
     for (int step = 0; step < z1 - z0; ++step) {
         const int z = p.back ? z1 - 1 - step : z0 + step;
         // the next plane (past the lattice: this one again, so that a cell's
@@ -175,8 +186,8 @@ xk_k_mass_quads(const uint32_t *__restrict__ src, uint32_t *__restrict__ dst, un
             if (r >= dup) {
                 sum += o.x + o.y + o.z + o.w;
                 if (PROJ) {
-                    cs[r][0] += colour(o.x) + (colour(o.y) << 16);
-                    cs[r][1] += colour(o.z) + (colour(o.w) << 16);
+                    add_shared(mine + 1024u * r, colour(o.x) + (colour(o.y) << 16));
+                    add_shared(mine + 1024u * r + 512u, colour(o.z) + (colour(o.w) << 16));
                 }
             }
             qp[r] = c;
@@ -194,8 +205,9 @@ xk_k_mass_quads(const uint32_t *__restrict__ src, uint32_t *__restrict__ dst, un
             if (r < dup) continue;
             // two columns an atomic: a sum stays below 2^32, so none carries
             unsigned long long *pair = (unsigned long long *)(proj + 4 * ((int64_t)(y + r) * p.P4 + xq));
-            atomicAdd(pair, (unsigned long long)(cs[r][0] >> 16) << 32 | (cs[r][0] & 0xFFFFu));
-            atomicAdd(pair + 1, (unsigned long long)(cs[r][1] >> 16) << 32 | (cs[r][1] & 0xFFFFu));
+            const uint32_t a = column[2 * r][threadIdx.x], b = column[2 * r + 1][threadIdx.x];
+            atomicAdd(pair, (unsigned long long)(a >> 16) << 32 | (a & 0xFFFFu));
+            atomicAdd(pair + 1, (unsigned long long)(b >> 16) << 32 | (b & 0xFFFFu));
         }
     }
     // one atomic a block: they all hit one address
