@@ -793,12 +793,14 @@ def lifecolor_line(args, dist):
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "peak_kind": peak_kind,
                          "traffic": committed_traffic("lifecolor"),
-                         "kernel": "xk_k_lifecolor per generation (it also writes the zoom-1 "
-                                   "uint8 frame)",
+                         "kernel": "xk_k_lifecolor, four generations a launch (it also writes "
+                                   "their zoom-1 uint8 frames)",
                          "algorithmic_bytes_per_generation": bytes_per_update * n,
                          "note": "B_alg = 35 B per cell-update (4 B state and 12 B colour read "
-                                 "and written, 3 B uint8 RGB pixel written)"},
-            "gpu_launches": gens * args.steps, "clocks": clk}
+                                 "and written, 3 B uint8 RGB pixel written); a launch reads and "
+                                 "writes state and colours once for four generations, so frac > 1 "
+                                 "is reference-format effective; traffic: DRAM bytes of one launch"},
+            "gpu_launches": args.steps * ((gens + 3) // 4), "clocks": clk}
     if dist.rank == 0:
         sys.path.insert(0, os.path.join(ROOT, "oracle"))
         import oracle as O
@@ -1016,7 +1018,7 @@ def noise_line(args, dist):
     clk = clocks.stop()
     dev_s = dist.max(sum(step_ms) / 1000.0)
     value = float(n) * gens * args.steps * dist.world / dev_s
-    # the viewer's form: 100 generations, each with its frame (one launch each)
+    # the viewer's form: 100 generations, each with its frame (one launch)
     model.set_viewport((W, H))
     fb = W * H * 3
     frames_dev = torch.empty(100 * fb, dtype=torch.uint8, device="cuda:%d" % dist.local)
@@ -1047,7 +1049,7 @@ def noise_line(args, dist):
                        "l2": "state + colours (29 MB) fit in L2"},
             "frames": {"value": float(n) * 100 / (frame_ms / 1000.0), "unit": "cell-updates/s",
                        "note": "100 generations, each with its 1920x1080 uint8 frame written by the "
-                               "step kernel (one launch per generation)"},
+                               "step kernel (one launch)"},
             "interpreter": {"value": float(n) * 100 / (vm_ms / 1000.0), "unit": "cell-updates/s",
                             "note": "the same model on the generic interpreter, 100 generations"},
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
@@ -1195,8 +1197,8 @@ def mass_line(args, dist):
                             "and copies none), every frame copied to page-locked host memory"},
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "peak_kind": peak_kind,
-                         "traffic": committed_traffic("mass_tma") if side == 256 else None,
-                         "kernel": "xk_k_mass_tma per generation (it also sums the column "
+                         "traffic": committed_traffic("mass_quads") if side == 256 else None,
+                         "kernel": "xk_k_mass_quads per generation (it also sums the column "
                                    "colours and writes the previous generation's frame)",
                          "algorithmic_bytes_per_generation": bytes_per_update * n,
                          "note": "B_alg = 12 B per cell-update (uint32 read + write, and the "
@@ -1357,8 +1359,8 @@ def life512_line(args, dist):
                               "note": "1000 calls of model.step(), one generation each"},
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "peak_kind": peak_kind,
-                         "traffic": committed_traffic("life_cluster"),
-                         "kernel": "xk_k_life_cluster (or the resident kernel, as tuned)",
+                         "traffic": committed_traffic("life_deep"),
+                         "kernel": "xk_k_life_deep (or another plan, as tuned)",
                          "note": "B_alg = 2 B per cell-update; the lattice stays in the "
                                  "shared memory of one CTA or of a thread-block cluster "
                                  "(whichever the first step's tuning found faster) for all "
