@@ -171,3 +171,48 @@ def test_random_programs(seed):
     got = _run(desc, (emit, absorb), init, col, False)
     assert np.array_equal(got[0], want[0])
     assert np.array_equal(got[1], want[1])
+
+
+@pytest.mark.parametrize("ty", [I32, U32])
+@pytest.mark.parametrize("swapped", [False, True])
+@pytest.mark.parametrize("again", ["never", "after", "overwritten"])
+def test_joined_operations(ty, swapped, again):
+    """Every pair of operations of which the second reads the first's result,
+    on either side, with that result read again, overwritten or dropped; the
+    sums of comparisons of masked values; one value stored to several planes."""
+    p = type("P", (), {"nregs": 16})()
+    p.consts = [vm.pack_value(v, ir.I32 if ty == I32 else ir.U32) for v in (3, 5, 7, 0)]
+    code = [(O["load"], U32, 0, 2, 0, 1, 0), (O["load"], U32, 1, 2, 1, 2, 0)]
+    code += [(O["const"], ty, 2 + k, k, 0, 0, 0) for k in range(4)]
+    code += [(O["cvt"], ty, 0, 0, U32, 0, 0), (O["cvt"], ty, 1, 1, U32, 0, 0), (O["mov"], ty, 6, 5, 0, 0, 0)]
+    ops = ["+", "*", "&", "|", "<<", ">>", "==", "<", "<=", "^", "-"]
+    for f in ops:
+        for s in ops:
+            dst = 7 if again == "overwritten" else 8
+            code.append((O[f], ty, 7, 0, 2 if f in ("<<", ">>") else 1, 0, 0))
+            a, b = (3, 7) if swapped and s not in ("<<", ">>") else (7, 3)
+            code.append((O[s], ty, dst, a, b, 0, 0))
+            code.append((O["^"], ty, 6, 6, dst, 0, 0))
+            if again == "after":
+                code.append((O["^"], ty, 6, 6, 7, 0, 0))
+            code.append((O["+"], ty, 6, 6, 4, 0, 0))
+    for k in range(6):
+        code.append((O["&"], ty, 7, k & 1, 2 + k % 3, 0, 0))
+        code.append((O["=="], ty, 7 if k & 2 else 8, 7, 2, 0, 0))
+        code.append((O["+"], ty, 6, 6, 7 if k & 2 else 8, 0, 0))
+    p.code = code + [(O["store"], U32, 0, 6, 0, 0, 0), (O["store"], U32, 0, 6, 0, 0, 0)]
+    e = type("P", (), {"nregs": 16, "consts": p.consts})()
+    e.code = [(O["load"], U32, 0, 0, 0, 0, 0), (O["const"], U32, 1, 0, 0, 0, 0)]
+    e.code += [(O["store"], U32, 0, 0, 1, 0, 0), (O["store"], U32, 0, 0, 3, 0, 0), (O["+"], U32, 2, 0, 1, 0, 0)]
+    e.code += [(O["store"], U32, 0, 2, 2, 0, 0), (O["store"], U32, 0, 2, 4, 0, 0)]
+    desc = nat.XkDesc()
+    desc.abi_version, desc.family, desc.ndim, desc.nbr = nat.XK_ABI_VERSION, nat.XK_FAMILY_VM, 2, 4
+    for d, size in enumerate((67, 5)):
+        desc.size[d] = size
+        desc.delta[2 * d][d], desc.delta[2 * d + 1][d] = 1, -1
+    desc.torus, desc.state_bytes, desc.color_kind = 1, 4, nat.XK_COLOR_PLAIN
+    r = np.random.RandomState(5)
+    init = r.choice(np.array(EDGE, dtype=np.uint64), 67 * 5).astype(np.uint32)
+    col = np.zeros(3 * init.size, dtype=np.int32)
+    want, got = _run(desc, (e, p), init, col, True), _run(desc, (e, p), init, col, False)
+    assert np.array_equal(got[0], want[0])

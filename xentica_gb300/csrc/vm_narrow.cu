@@ -16,13 +16,19 @@
 // operation's dispatch covers the next one's operand loads; an operand that
 // is its result is taken from registers.
 //
+// An operation whose result only the next one reads is joined with it (63
+// pairs of the common integer operations, and the addition of a comparison of
+// a masked value), stores of one value to several planes are one.
+//
 // Bound by the latency of an operation (fetch, dispatch, shared memory: about
-// 250 cycles a warp, the same at three warps a scheduler as at one).  640 x
-// 360 cells, 65 absorb operations (123 as loaded) and 11 of emit, a frame a
-// generation: 18.3 us, against 81.6 us with vm.cu's 64-bit registers in local
-// memory and one cell a thread.  Measured and not kept: eight cells a thread
-// (16.8 against 16.7 us on such a program, 108 against 107 at 1920 x 1080),
-// the code in shared memory (17.8), operand loads behind the dispatch (19.9).
+// 240 cycles a warp, 360 of a pair, the same at three warps a scheduler as at
+// one).  640 x 360 cells, 65 absorb operations (123 as loaded) and 11 of emit
+// before the joins, a frame a generation: 16.0 us, 18.3 without them, against
+// 81.6 us with vm.cu's 64-bit registers in local memory and one cell a thread.
+// Measured and not kept: eight cells a thread (16.8 against 16.7 us on such a
+// program, 108 against 107 at 1920 x 1080), the code in shared memory (17.8),
+// operand loads behind the dispatch (19.9), the third operand loaded ahead as
+// the others are (16.9 against 16.7 before stores were joined).
 #include <string.h>
 
 #include <algorithm>
@@ -37,21 +43,30 @@ enum {
     N_LTS, N_LTU, N_LES, N_LEU, N_EQ, N_NE,
     N_FADD, N_FSUB, N_FMUL, N_FDIV, N_FLT, N_FLE, N_FEQ, N_FNE,
     N_NEG, N_NOT, N_ABSS, N_FNEG, N_FABS, N_SEL, N_BOOL, N_I2F, N_U2F, N_F2S, N_F2U, N_F2B, N_POPC, N_MOV,
-    N_PARAM, N_LOAD, N_STORE, N_COLOR
+    N_PARAM, N_LOAD, N_STORE, N_COLOR,
+    N_STORES,                   // one value to several planes (imm: their mask), as emit copies a cell
+    N_COUNT,                    // ((a & b) == c) + d: one more neighbour in a state
+    N_PAIR                      // two operations in one: N_PAIR + first * VN_SECONDS + second
 };
-enum { NF_A = 1, NF_B = 2, NF_C = 4, NF_STORE = 8 };   // operands and result an operation has
+// An operation whose result only the next one reads joins it: (a first b)
+// second c, for these (second's operands swapped where it commutes)
+constexpr int VN_FIRST[] = {N_ADD, N_MUL, N_AND, N_OR, N_SHRU, N_SHL, N_EQ, N_LTU, N_LTS};
+constexpr int VN_SECOND[] = {N_ADD, N_MUL, N_AND, N_OR, N_EQ, N_SHRU, N_SHL};
+constexpr int VN_SECONDS = 7;
+enum { NF_A = 1, NF_B = 2, NF_C = 4, NF_STORE = 8, NF_D = 16 };   // operands and result an operation has
 #define XK_VN_CONST 0x8000     // a slot number with this bit is a constant's
 
 // translation: loads: a = kind (0 own cell, 1 neighbour), c = plane, imm = the
 // neighbour's offsets + 1, two bits an axis; stores: imm = plane; parameters:
-// a = slot.
+// a = slot; a fourth operand: imm.
 struct XkVnOp {
     uint16_t op, flags, dst, a, b, c;
     uint32_t imm;
 };
 
 // What the kernel reads.  Loads: c = kind (0 own cell, 1 neighbour), imm as
-// above; stores and loads: plane; parameters: c = slot.
+// above; stores and loads: plane (elsewhere a fourth operand); parameters: c =
+// slot.
 struct XkVnCode {
     uint16_t dst, a, b, c, op, plane;
     uint32_t imm;
@@ -135,6 +150,28 @@ __device__ __forceinline__ void vn_sts(uint32_t at, const uint4 &v)
     asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" : : "r"(at), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w)
                  : "memory");
 }
+
+template <int OP>
+__device__ __forceinline__ uint32_t vn_do(uint32_t x, uint32_t y)
+{
+    return OP == N_ADD ? x + y : OP == N_MUL ? x * y : OP == N_AND ? x & y : OP == N_OR ? x | y
+           : OP == N_SHRU ? x >> (y & 31u) : OP == N_SHL ? x << (y & 31u) : OP == N_EQ ? (uint32_t)(x == y)
+           : OP == N_LTU ? (uint32_t)(x < y) : (uint32_t)((int32_t)x < (int32_t)y);
+}
+
+template <int FIRST, int SECOND>
+__device__ __forceinline__ uint4 vn_pair(const uint4 &a, const uint4 &b, const uint4 &c)
+{
+    constexpr int F = VN_FIRST[FIRST], S = VN_SECOND[SECOND];
+    return make_uint4(vn_do<S>(vn_do<F>(a.x, b.x), c.x), vn_do<S>(vn_do<F>(a.y, b.y), c.y),
+                      vn_do<S>(vn_do<F>(a.z, b.z), c.z), vn_do<S>(vn_do<F>(a.w, b.w), c.w));
+}
+
+#define XK_VN_PAIR(F, S)                                                                                     \
+    case N_PAIR + (F) * VN_SECONDS + (S): acc = vn_pair<F, S>(va, vb, get(o.y >> 16)); break;
+#define XK_VN_PAIRS(F)                                                                                       \
+    XK_VN_PAIR(F, 0) XK_VN_PAIR(F, 1) XK_VN_PAIR(F, 2) XK_VN_PAIR(F, 3) XK_VN_PAIR(F, 4) XK_VN_PAIR(F, 5)    \
+    XK_VN_PAIR(F, 6)
 
 #define XK_VN_ONE(f, expr)                                                                                   \
     {                                                                                                        \
@@ -364,6 +401,33 @@ xk_k_vm_narrow(uint8_t *__restrict__ fld, int32_t *__restrict__ col, const __gri
             }
             break;
         }
+        case N_STORES: {
+            const uint32_t v[4] = {va.x, va.y, va.z, va.w};
+            for (uint32_t left = o.w; left != 0; left &= left - 1) {
+                uint8_t *plane = fld + (int64_t)p.n * (__ffs((int)left) - 1) * ESZ;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const uint32_t i = w0 + 32u * k + lane;
+                    if (i < p.n) vn_st<ESZ>(plane, i, v[k]);
+                }
+            }
+            break;
+        }
+        case N_COUNT: {
+            const uint4 vc = get(o.y >> 16), vd = get(o.z >> 16);
+            acc = make_uint4(((va.x & vb.x) == vc.x) + vd.x, ((va.y & vb.y) == vc.y) + vd.y,
+                             ((va.z & vb.z) == vc.z) + vd.z, ((va.w & vb.w) == vc.w) + vd.w);
+            break;
+        }
+        XK_VN_PAIRS(0)
+        XK_VN_PAIRS(1)
+        XK_VN_PAIRS(2)
+        XK_VN_PAIRS(3)
+        XK_VN_PAIRS(4)
+        XK_VN_PAIRS(5)
+        XK_VN_PAIRS(6)
+        XK_VN_PAIRS(7)
+        XK_VN_PAIRS(8)
         default: break;
         }
         put(dst, acc);                           // operations without a result have a slot nothing reads
@@ -707,6 +771,75 @@ void Translator::one(const xk_vm_ins &in)
     }
 }
 
+// Operations joined with the next one where nothing else reads their result:
+// the slot is the next one's result too, or is written before it is read
+// again.  Stores of one value one after another become one.
+void join(std::vector<XkVnOp> &body)
+{
+    auto reads = [](const XkVnOp &o, int slot) {
+        return ((o.flags & NF_A) && o.a == slot) || ((o.flags & NF_B) && o.b == slot) ||
+               ((o.flags & NF_C) && o.c == slot) || ((o.flags & NF_D) && (int)o.imm == slot);
+    };
+    auto alone = [&](size_t i) {        // only operation i + 1 reads operation i's result
+        const int slot = body[i].dst;
+        if ((body[i + 1].flags & NF_STORE) && body[i + 1].dst == slot) return true;
+        for (size_t k = i + 2; k < body.size(); ++k) {
+            if (reads(body[k], slot)) return false;
+            if ((body[k].flags & NF_STORE) && body[k].dst == slot) return true;
+        }
+        return true;
+    };
+    auto find = [](const int *ops, int n, int op) { return (int)(std::find(ops, ops + n, op) - ops); };
+    // the operand of o beside slot (once an operand, first or in an operation
+    // that commutes), or -1
+    auto other = [](const XkVnOp &o, int slot) {
+        if (o.a == slot && o.b != slot) return (int)o.b;
+        const bool swaps = o.op == N_ADD || o.op == N_MUL || o.op == N_AND || o.op == N_OR || o.op == N_EQ;
+        return o.b == slot && o.a != slot && swaps ? (int)o.a : -1;
+    };
+    constexpr int FIRSTS = sizeof(VN_FIRST) / sizeof(int);
+    std::vector<XkVnOp> out;
+    for (size_t i = 0; i < body.size(); ++i) {
+        XkVnOp o = body[i];
+        const int f = find(VN_FIRST, FIRSTS, o.op);
+        if (f < FIRSTS && i + 1 < body.size()) {
+            const XkVnOp &p = body[i + 1];
+            const int s = find(VN_SECOND, VN_SECONDS, p.op), c = s < VN_SECONDS ? other(p, o.dst) : -1;
+            if (c >= 0 && alone(i)) {
+                // an addition to the comparison of a masked value
+                const int d = o.op == N_AND && p.op == N_EQ && i + 2 < body.size() && body[i + 2].op == N_ADD
+                                  ? other(body[i + 2], p.dst) : -1;
+                o.c = (uint16_t)c;
+                o.flags |= NF_C;
+                if (d >= 0 && alone(i + 1)) {
+                    o.op = N_COUNT;
+                    o.imm = (uint32_t)d;
+                    o.flags |= NF_D;
+                    o.dst = body[i + 2].dst;
+                    i += 2;
+                } else {
+                    o.op = (uint16_t)(N_PAIR + f * VN_SECONDS + s);
+                    o.dst = p.dst;
+                    ++i;
+                }
+            }
+        }
+        if (o.op == N_STORE && o.imm < 32) {
+            uint32_t planes = 1u << o.imm;
+            size_t k = i + 1;
+            for (; k < body.size() && body[k].op == N_STORE && body[k].a == o.a && body[k].imm < 32; ++k)
+                planes |= 1u << body[k].imm;
+            if (k > i + 1) {
+                o.op = N_STORES;
+                o.imm = planes;
+                i = k - 1;
+            }
+        }
+        out.push_back(o);
+    }
+    body.swap(out);
+}
+
 }  // namespace
 
 bool xk_vm_translate(const xk_vm_ins *code, int ncode, const uint64_t *consts, int nregs, const VmGeo &g,
@@ -745,6 +878,7 @@ bool xk_vm_translate(const xk_vm_ins *code, int ncode, const uint64_t *consts, i
         }
     }
     if (slots >= XK_VN_CONST) return false;
+    join(body);
     // slots that are never used drop out
     std::vector<int> used(slots, 0);
     auto mark = [&](const XkVnOp &o) {
@@ -752,6 +886,7 @@ bool xk_vm_translate(const xk_vm_ins *code, int ncode, const uint64_t *consts, i
         if ((o.flags & NF_A) && !(o.a & XK_VN_CONST)) used[o.a] = 1;
         if ((o.flags & NF_B) && !(o.b & XK_VN_CONST)) used[o.b] = 1;
         if ((o.flags & NF_C) && !(o.c & XK_VN_CONST)) used[o.c] = 1;
+        if ((o.flags & NF_D) && !(o.imm & XK_VN_CONST)) used[o.imm] = 1;
     };
     for (const XkVnOp &o : head) mark(o);
     for (const XkVnOp &o : body) mark(o);
@@ -762,6 +897,7 @@ bool xk_vm_translate(const xk_vm_ins *code, int ncode, const uint64_t *consts, i
         if ((o.flags & NF_A) && !(o.a & XK_VN_CONST)) o.a = (uint16_t)used[o.a];
         if ((o.flags & NF_B) && !(o.b & XK_VN_CONST)) o.b = (uint16_t)used[o.b];
         if ((o.flags & NF_C) && !(o.c & XK_VN_CONST)) o.c = (uint16_t)used[o.c];
+        if ((o.flags & NF_D) && !(o.imm & XK_VN_CONST)) o.imm = (uint32_t)used[o.imm];
     };
     out->nloads = (int)head.size();
     out->nops = (int)(head.size() + body.size());
@@ -798,7 +934,9 @@ bool xk_vm_translate(const xk_vm_ins *code, int ncode, const uint64_t *consts, i
         c.a = place(o.flags & NF_A ? o.a : XK_VN_CONST);
         c.b = place(o.flags & NF_B ? o.b : XK_VN_CONST);
         c.c = place(o.flags & NF_C ? o.c : XK_VN_CONST);
+        if (o.flags & NF_D) c.plane = place((int)o.imm);
         if (o.op == N_STORE) c.plane = (uint16_t)o.imm;
+        if (o.op == N_STORES) c.imm = o.imm;
         if (o.op == N_PARAM) c.c = o.a;
         if (o.op == N_LOAD) {
             c.c = o.a;
