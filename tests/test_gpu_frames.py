@@ -140,3 +140,27 @@ def test_evolife_frames_match_oracle_render():
             if model.is_constant("SMOOTH_FACTOR") else 0
         img = O.render(topo, col, 131, 103, smooth=smooth).astype(np.uint8)
         assert np.array_equal(frames[g], img), "frame %d" % g
+
+
+@pytest.mark.parametrize("size", [(97, 61), (64, 40), (131, 70)])
+@pytest.mark.parametrize("view", [(97, 61, 1, 0, 0), (50, 33, 1, 7, -3), (200, 90, 3, -5, 11), (31, 200, 2, 95, 60)])
+def test_pictures_of_colours_that_follow_from_the_state(size, view):
+    """Rendered from the packed cells, the same picture as from the colours
+    written out; colours that have been shown stay with an upload of cells."""
+    exp = type("E", (GOLExperiment2, ), {"size": size})
+    model = GameOfLife(exp)
+    n = model.cells_num
+    cells = (np.random.RandomState(size[0]).random_sample(n) < 0.4).astype(np.uint8)
+    model.gpu.load(cells, np.zeros(3 * n, dtype=np.int32))
+    model.gpu.step(3)
+    w, h, zoom, dx, dy = view
+    model.set_viewport((w, h))
+    packed = model.gpu.render(w, h, zoom, dx, dy).copy()
+    assert packed.any()
+    other = np.ascontiguousarray(1 - cells)
+    nat.check(model.gpu._lib.xk_upload(model.gpu._handle, nat.ptr(other), n), "xk_upload")
+    assert np.array_equal(model.gpu.render(w, h, zoom, dx, dy), packed)
+    model.gpu.load(cells, np.zeros(3 * n, dtype=np.int32))
+    model.gpu.step(3)
+    model.gpu.arrays.colors.get()
+    assert np.array_equal(model.gpu.render(w, h, zoom, dx, dy), packed)

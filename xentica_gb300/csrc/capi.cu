@@ -207,6 +207,7 @@ struct xk_model {
     VmGeo vg;
     int hf = 0;                  // colour is a function of the state alone
     int derived = 0;             // colours currently implied by the state
+    int shown = 0;               // ... and a picture of them has been rendered
     int uploaded = 0;
     // xk_step_frames to host memory: device frame ring and its copy stream
     uint8_t *ring = nullptr;
@@ -674,11 +675,18 @@ extern "C" void xk_model_destroy(xk_model *m)
     free_model(m);
 }
 
+static int materialize_colors(xk_model *m);
+
 extern "C" int xk_upload(xk_model *m, const void *host_main, int64_t ncells)
 {
     XK_REQUIRE(m && host_main, XK_ERR_ARG, "xk_upload: null argument");
     XK_REQUIRE(ncells == m->n, XK_ERR_ARG, "xk_upload: %lld cells given, model has %lld",
                (long long)ncells, (long long)m->n);
+    if (m->derived && m->shown) {
+        // colours that have been shown stay until the next step
+        int rc = materialize_colors(m);
+        if (rc != XK_OK) return rc;
+    }
     const int esz = m->d.state_bytes;
     if (m->layout == LAYOUT_CELLS64 || m->layout == LAYOUT_MASS || m->layout == LAYOUT_VM ||
         m->layout == LAYOUT_LCOLOR || m->layout == LAYOUT_NOISE || m->layout == LAYOUT_GRAVITY) {
@@ -777,6 +785,9 @@ extern "C" int xk_download(xk_model *m, void *host_main, int64_t ncells)
 }
 
 // write the colours implied by the state into m->col
+// what a derived colour is its table's value times
+static int color_scale(const xk_model *m) { return m->d.color_kind == XK_COLOR_MOVING_AVERAGE ? m->d.smooth : 1; }
+
 static int materialize_colors(xk_model *m)
 {
     if (m->layout == LAYOUT_VM || m->layout == LAYOUT_LCOLOR || m->layout == LAYOUT_NOISE ||
@@ -787,11 +798,10 @@ static int materialize_colors(xk_model *m)
         return XK_OK;
     }
     if (!m->derived) return XK_OK;
-    const int smooth = m->d.color_kind == XK_COLOR_MOVING_AVERAGE ? m->d.smooth : 1;
     if (bits_layout(m))
-        XK_CUDA(xk_life_colors(m->bits[m->cur], m->col, m->lg, m->lut, smooth, m->stream));
+        XK_CUDA(xk_life_colors(m->bits[m->cur], m->col, m->lg, m->lut, color_scale(m), m->stream));
     else
-        XK_CUDA(xk_nd_colors(m->bytes[m->cur], m->col, m->n, m->lut, smooth, m->stream));
+        XK_CUDA(xk_nd_colors(m->bytes[m->cur], m->col, m->n, m->lut, color_scale(m), m->stream));
     m->derived = 0;
     return XK_OK;
 }
@@ -1079,7 +1089,10 @@ static int step_enqueue(xk_model *m, int64_t first, int64_t count, uint8_t *fram
         }
     }
     // history-free colours are implied by the state from here on
-    if (colors_free && m->d.color_kind != XK_COLOR_NONE) m->derived = 1;
+    if (colors_free && m->d.color_kind != XK_COLOR_NONE) {
+        m->derived = 1;
+        m->shown = 0;
+    }
     return XK_OK;
 }
 
@@ -1258,8 +1271,6 @@ static int render_enqueue(xk_model *m, void *img, bool bytes, int32_t width, int
                                    m->stream));
         return XK_OK;
     }
-    int rc = materialize_colors(m);
-    if (rc != XK_OK) return rc;
     RenderGeo g;
     memset(&g, 0, sizeof(g));
     g.ndim = m->d.ndim;
@@ -1267,6 +1278,14 @@ static int render_enqueue(xk_model *m, void *img, bool bytes, int32_t width, int
     g.a1 = m->d.proj_axis1;
     for (int i = 0; i < m->d.ndim; ++i) g.size[i] = m->d.size[i];
     g.smooth = m->d.render_smooth;
+    if (m->derived && bits_layout(m) && xk_render_is_2d(g, width, height, zoom)) {
+        XK_CUDA(xk_render_bits(m->bits[m->cur], img, bytes, m->lg, m->lut, color_scale(m), g, width, height, zoom, dx,
+                               dy, m->stream));
+        m->shown = 1;
+        return XK_OK;
+    }
+    int rc = materialize_colors(m);
+    if (rc != XK_OK) return rc;
     if (bytes)
         XK_CUDA(xk_render_colors_u8(m->col, (uint8_t *)img, g, width, height, zoom, dx, dy, m->stream));
     else
