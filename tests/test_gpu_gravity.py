@@ -153,3 +153,38 @@ def test_special_gravities_vs_oracle(cls, border):
     g, w = [(a >> np.uint64(24)).astype(np.uint32).view(np.float32) for a in (got, want)]
     assert np.isnan(w).any() and np.isinf(w).any()
     assert np.array_equal(g, w, equal_nan=True)
+
+
+# two windows of 60 x 30 an SM and more, rows of a multiple of four: four cells
+# a thread (the sizes above run one); last windows of one quad, of one row,
+# one window wide, one high
+@pytest.mark.parametrize("size", [(1084, 541), (1080, 511), (4, 9150), (18420, 1), (1196, 480)])
+@pytest.mark.parametrize("cls,border", [(GraviCowboys, None), (GraviCowboysStatic, STATIC)])
+def test_quads_vs_oracle(cls, border, size):
+    """Cells, colours and frames, then NaN, infinite and negative-zero
+    gravities among ties (a NaN's bits compared as NaN)."""
+    n = size[0] * size[1]
+    cells = random_cells(n, n, energies=8)
+    model, colors = _model(cls, size, cells, n)
+    model.set_viewport(size)
+    topo = O.Topology(size, "moore", border)
+    fld = topo.field(cells, np.uint64)
+    col = colors.copy()
+    frames = model.step_frames(3)
+    for g in range(3):
+        O.gravity_run(topo, fld, col, 1, color=O._color(True, 255, 255, 1))
+        assert np.array_equal(frames[g], O.render(topo, col, size[0], size[1], smooth=1).astype(np.uint8)), g
+    assert np.array_equal(model.gpu.arrays.cells.get()[:n], fld[:n])
+    assert np.array_equal(model.gpu.arrays.colors.get(), col)
+    rng = np.random.RandomState(n)
+    special = np.array([np.nan, np.inf, -np.inf, -0.0, 0.0], dtype=np.float32).view(np.uint32).astype(np.uint64)
+    cells = np.where(rng.random_sample(n) < 0.01,
+                     (cells & np.uint64(0xFFFFFF)) | special[rng.randint(0, 5, n)] << np.uint64(24), cells)
+    model, _ = _model(cls, size, cells, 3)
+    fld = topo.field(cells, np.uint64)
+    model.gpu.step(1)
+    O.gravity_run(topo, fld, np.zeros(3 * n, dtype=np.int32), 1)
+    got, want = model.gpu.arrays.cells.get()[:n], fld[:n]
+    assert np.array_equal(got & np.uint64(0xFFFFFF), want & np.uint64(0xFFFFFF))
+    g, w = [(a >> np.uint64(24)).astype(np.uint32).view(np.float32) for a in (got, want)]
+    assert np.array_equal(g, w, equal_nan=True)

@@ -558,10 +558,10 @@ xk_k_evolife(const uint64_t *__restrict__ src, uint64_t *__restrict__ dst, int32
     const bool fades = p.color_kind == XK_COLOR_MOVING_AVERAGE;
     const int64_t first = 3 * ((int64_t)y * p.W + x0);      // the row's first colour word
     if (fades && row_in)
-        xk_col_fetch<true, XK_EVO_TX>(T.col[r], col, first, width, 3 * (int64_t)p.W * p.H, q);
-    xk_copy_async<16>(&T.slots[tid], p.slots + tid);
+        xk_col_fetch<XK_EVO_TX>(T.col[r], col, first, width, q);
+    xk_copy_async16(&T.slots[tid], p.slots + tid);
     if (!POS)
-        for (int k = tid; k < 360; k += 256) xk_copy_async<16>(&T.hues[k], p.hues + k);
+        for (int k = tid; k < 360; k += 256) xk_copy_async16(&T.hues[k], p.hues + k);
     uint64_t own[4], halo[4];
     xk_evo_get(src + (int64_t)(row_in ? y : y % p.H) * p.W, x, p.W, own);
     const int h = tid - 2 * XK_EVO_QX;              // the halo: two rows, then two quads a row
@@ -629,7 +629,7 @@ xk_k_evolife(const uint64_t *__restrict__ src, uint64_t *__restrict__ dst, int32
     }
     int *mine = (int *)T.col[r] + 12 * q;
     int c[12];
-    if (fades) xk_col_read<true>(mine, c);
+    if (fades) xk_col_read(mine, c);
     // genome_crossover(main, 18, *genomes, max_genes, mutation_prob), step by
     // step for the four cells.  With no parent, every gene is 0 (no winner,
     // and a mutation needs a gene that some parent has).
@@ -710,9 +710,9 @@ xk_k_evolife(const uint64_t *__restrict__ src, uint64_t *__restrict__ dst, int32
                      "l"(out[2]), "l"(out[3])
                      : "memory");
     if (p.color_kind == XK_COLOR_NONE) return;
-    xk_col_write<true>(mine, c);
+    xk_col_write(mine, c);
     __syncwarp();
-    if (row_in) xk_col_store<true, XK_EVO_TX>(T.col[r], col, first, width, q);
+    if (row_in) xk_col_store<XK_EVO_TX>(T.col[r], col, first, width, q);
     if (!p.frame) return;
     uint32_t b[3];
     xk_pixels4(c, mine, p.small != 0, p.frame_smooth, b);

@@ -33,12 +33,11 @@
 // own 48 bytes ran a generation in 19.0 us, this in 17.2, before the pixels of
 // colours beyond 2^24 moved out of line).
 //
-// 64 frames of 1920 x 1080: 1067 us, against 1382 of one cell a thread (its
+// 64 frames of 1920 x 1080: 1080 us, against 1410 of one cell a thread (its
 // 274 instructions a cell issued at 65 %; now 187, at 60 % of 42 % of the
 // warps: what is left to hide is the latency of one short launch a
-// generation).  Where rows do not start on 16 bytes, states move in 8-byte
-// loads and colours pass shared memory by words: 1394 us at 1919 x 1079
-// (1414 before), 343 at 301 x 203 (465).
+// generation).  Small lattices, and rows that do not start on 16
+// bytes, run one cell a thread (below).
 #include "xk_internal.cuh"
 
 #include "frame.cuh"
@@ -139,7 +138,7 @@ static __device__ __noinline__ float xk_gc_lowest(const float *at)
     return m;
 }
 
-template <bool TORUS, bool ALIGNED>
+template <bool TORUS>
 __global__ void __launch_bounds__(XK_GC_THREADS, 3)
 xk_k_gravity(const uint64_t *__restrict__ src, uint64_t *__restrict__ dst, int32_t *__restrict__ col,
              GravParams p)
@@ -176,8 +175,7 @@ xk_k_gravity(const uint64_t *__restrict__ src, uint64_t *__restrict__ dst, int32
         for (int r = half; r < XK_GC_IY; r += HALVES) {
             const int gy = y0 + 1 + r;
             if (gy < p.H)
-                xk_col_fetch<ALIGNED, XK_GC_IX>(T.col[r], col, 3 * ((int64_t)gy * p.W + x0 + 2), width,
-                                                3 * (int64_t)p.W * p.H, q);
+                xk_col_fetch<XK_GC_IX>(T.col[r], col, 3 * ((int64_t)gy * p.W + x0 + 2), width, q);
         }
     uint64_t v[ROWS][2];
 #pragma unroll
@@ -195,14 +193,9 @@ xk_k_gravity(const uint64_t *__restrict__ src, uint64_t *__restrict__ dst, int32
         }
         const uint64_t *row = src + (int64_t)gy * p.W;
         if (r < XK_GC_WY + 2) {
-            if (ALIGNED) {
-                const ulonglong2 w = __ldg((const ulonglong2 *)(row + gx[0]));
-                v[i][0] = w.x;
-                v[i][1] = w.y;
-            } else {
-                v[i][0] = __ldg(row + gx[0]);
-                v[i][1] = __ldg(row + gx[1]);
-            }
+            const ulonglong2 w = __ldg((const ulonglong2 *)(row + gx[0]));
+            v[i][0] = w.x;
+            v[i][1] = w.y;
         }
         if (!TORUS) {
             if (!(xin[0] && yin)) v[i][0] = p.border;
@@ -357,29 +350,15 @@ xk_k_gravity(const uint64_t *__restrict__ src, uint64_t *__restrict__ dst, int32
             energy[k] = TORUS ? newe + received : (newe + received) & 0xFFFFu;
             out[k] = (uint64_t)(energy[k] & 4095u) | (uint64_t)newe << 12 | (uint64_t)__float_as_uint(g[k]) << 24;
         }
-        if (in) {
-            if (ALIGNED) {
-                asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(dst + i), "l"(out[0]), "l"(out[1]),
-                             "l"(out[2]), "l"(out[3])
-                             : "memory");
-            } else if (ox + 4 > p.W) {
-#pragma unroll
-                for (int k = 0; k < 3; ++k)
-                    if (ox + k < p.W) dst[i + k] = out[k];
-            } else if ((i & 1) == 0) {
-                *(ulonglong2 *)(dst + i) = make_ulonglong2(out[0], out[1]);
-                *(ulonglong2 *)(dst + i + 2) = make_ulonglong2(out[2], out[3]);
-            } else {
-                dst[i] = out[0];
-                *(ulonglong2 *)(dst + i + 1) = make_ulonglong2(out[1], out[2]);
-                dst[i + 3] = out[3];
-            }
-        }
+        if (in)
+            asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(dst + i), "l"(out[0]), "l"(out[1]),
+                         "l"(out[2]), "l"(out[3])
+                         : "memory");
         if (!colours) continue;
         const int64_t first = 3 * ((int64_t)gy * p.W + x0 + 2);
-        int *mine = (int *)T.col[top] + (ALIGNED ? 0 : (int)(first & 3)) + 12 * min(q, 14);
+        int *mine = (int *)T.col[top] + 12 * min(q, 14);
         int c[12];
-        xk_col_read<ALIGNED>(mine, c);
+        xk_col_read(mine, c);
         __syncwarp();
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
@@ -388,16 +367,167 @@ xk_k_gravity(const uint64_t *__restrict__ src, uint64_t *__restrict__ dst, int32
             c[3 * k + 1] = xk_fade(gg, c[3 * k + 1], p.fade_in, p.neg_fade_out);
             c[3 * k + 2] = xk_fade(gg, c[3 * k + 2], p.fade_in, p.neg_fade_out);
         }
-        if (in) xk_col_write<ALIGNED>(mine, c);
+        if (in) xk_col_write(mine, c);
         __syncwarp();
-        if (row_in) xk_col_store<ALIGNED, XK_GC_IX>(T.col[r], col, first, width, q);
+        if (row_in) xk_col_store<XK_GC_IX>(T.col[r], col, first, width, q);
         if (!p.frame) continue;
         uint32_t b[3];
         xk_pixels4(c, mine, p.frame_smooth <= 1 && xk_px_small12(c), p.frame_smooth, b);
         const int left = lane & 16;                     // the row's half warp
         uint8_t *at = p.frame + 3 * i;
         xk_store_px4(at, b, lane, left, row_in ? left + width / 4 - 1 : -1);
-        if (!ALIGNED && in && ox + 4 > p.W) xk_store_px_rest(at, b, p.W - ox);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// One cell a thread on 32 x 32 tiles with a halo of two: lattices of too few
+// windows to fill the chip, and rows that do not start on 16 bytes
+// (xk_gravity_step's rule).
+
+// the Moore deltas in the reference's order (x, y): (-1,-1) (-1,0) (-1,1)
+// (0,-1) (0,1) (1,-1) (1,0) (1,1); neighbour 7 - k points back along k
+__device__ __forceinline__ int xk_gc_dx(int k) { return k < 3 ? -1 : k < 5 ? 0 : 1; }
+__device__ __forceinline__ int xk_gc_dy(int k) { return (k == 0 || k == 3 || k == 5) ? -1 : (k == 1 || k == 6) ? 0 : 1; }
+
+// the quotient of any field (zeros keep their sign)
+__device__ __forceinline__ float xk_gc_mean_any(float f)
+{
+    float s;
+    if (xk_gc_mean(f, s) && fabsf(f) >= 0x1p-60f && fabsf(f) <= 0x1p+120f) return s;
+    return f == 0.0f ? f : xk_gc_mean_f64(f);
+}
+
+#define XK_GC1_TX 32
+#define XK_GC1_TY 32            // rows of a tile; each of the 8 warps runs four of them
+
+struct GravTileOne {
+    float g[XK_GC1_TY + 4][XK_GC1_TX + 4];        // gravities, halo of two
+    uint32_t e[XK_GC1_TY + 4][XK_GC1_TX + 4];     // energies
+    // emitted: .x units sent (bit k: to neighbour k) | new_energy << 8, .y the
+    // bits of the gravity every buffer carries (one 64-bit load in absorb)
+    uint2 x[XK_GC1_TY + 2][XK_GC1_TX + 2];
+};
+
+// emit of the cell at tile position (y, x): the units go to the neighbours of
+// the lowest gravity in neighbour order, one each while energy lasts, i.e. to
+// the first min(energy, ties) of them
+__device__ __forceinline__ void xk_gc_emit(GravTileOne &T, int y, int x, int ey, int ex)
+{
+    const uint32_t energy = T.e[y][x];
+    float gk[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) gk[k] = T.g[y + xk_gc_dy(k)][x + xk_gc_dx(k)];
+    float m = gk[0];
+#pragma unroll
+    for (int k = 1; k < 8; ++k) m = m < gk[k] ? m : gk[k];
+    const float lowest = __fadd_rn(0.0f, m);
+    uint32_t ties = 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) ties |= (uint32_t)(lowest == gk[k]) << k;
+    uint32_t mask = ties;
+    if (energy < (uint32_t)__popc(ties)) {       // energy < 8: only its first set bits
+        uint32_t rest = ties;
+        mask = 0;
+        for (uint32_t j = 0; j < energy; ++j) {
+            const uint32_t low = rest & (0u - rest);
+            mask |= low;
+            rest ^= low;
+        }
+    }
+    T.x[ey][ex] = make_uint2(mask | (energy - (uint32_t)__popc(mask)) << 8,
+                             __float_as_uint(__fadd_rn(T.g[y][x], (float)energy)));
+}
+
+template <bool TORUS>
+__global__ void __launch_bounds__(XK_GC_THREADS)
+xk_k_gravity_one(const uint64_t *__restrict__ src, uint64_t *__restrict__ dst, int32_t *__restrict__ col,
+             GravParams p)
+{
+    __shared__ GravTileOne T;
+    const int tid = threadIdx.y * XK_GC1_TX + threadIdx.x;
+    const int x0 = blockIdx.x * XK_GC1_TX, y0 = blockIdx.y * XK_GC1_TY;
+    xk_grid_dep_wait();                 // launched as a dependent of the previous generation
+    for (int e = tid; e < (XK_GC1_TY + 4) * (XK_GC1_TX + 4); e += XK_GC_THREADS) {
+        const int sy = e / (XK_GC1_TX + 4), sx = e % (XK_GC1_TX + 4);
+        int gx = x0 + sx - 2, gy = y0 + sy - 2;
+        uint64_t v;
+        if (TORUS) {
+            if ((unsigned)gx >= (unsigned)p.W) { gx %= p.W; if (gx < 0) gx += p.W; }
+            if ((unsigned)gy >= (unsigned)p.H) { gy %= p.H; if (gy < 0) gy += p.H; }
+            v = __ldg(src + (int64_t)gy * p.W + gx);
+        } else {
+            v = (gx >= 0 && gx < p.W && gy >= 0 && gy < p.H) ? __ldg(src + (int64_t)gy * p.W + gx) : p.border;
+        }
+        T.g[sy][sx] = xk_gc_grav(v);
+        T.e[sy][sx] = (uint32_t)v & 4095u;
+    }
+    __syncthreads();
+    for (int e = tid; e < (XK_GC1_TY + 2) * (XK_GC1_TX + 2); e += XK_GC_THREADS) {
+        const int ey = e / (XK_GC1_TX + 2), ex = e % (XK_GC1_TX + 2);
+        xk_gc_emit(T, ey + 1, ex + 1, ey, ex);   // off-board positions are never read
+    }
+    __syncthreads();
+    const int gx = x0 + threadIdx.x;
+    if (gx >= p.W) return;
+#pragma unroll
+    for (int r = 0; r < XK_GC1_TY / 8; ++r) {
+        const int ly = threadIdx.y + 8 * r, gy = y0 + ly;
+        if (gy >= p.H) return;
+        const int ty = ly + 1, tx = threadIdx.x + 1;
+        uint32_t got = 0, received = 0;
+        float gk[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const int dx = xk_gc_dx(k), dy = xk_gc_dy(k);
+            const bool on = TORUS || ((unsigned)(gx + dx) < (unsigned)p.W && (unsigned)(gy + dy) < (unsigned)p.H);
+            if (on) {
+                const uint2 w = T.x[ty + dy][tx + dx];
+                got |= w.x & (1u << (7 - k));   // the unit neighbour k sent back along k
+                gk[k] = __uint_as_float(w.y);
+            } else {
+                received += (uint32_t)p.border & 4095u;
+                gk[k] = xk_gc_grav(p.border);
+            }
+        }
+        received += (uint32_t)__popc(got);
+        float field = 0.0f;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) field = __fadd_rn(field, gk[k]);
+        const uint32_t newe = T.x[ty][tx].x >> 8;
+        const uint32_t energy = (newe + received) & 0xFFFFu;
+        const float g = xk_gc_mean_any(field);
+        const int64_t i = (int64_t)gy * p.W + gx;
+        dst[i] = (uint64_t)(energy & 4095u) | (uint64_t)newe << 12 | (uint64_t)__float_as_uint(g) << 24;
+        if (p.color_kind == XK_COLOR_NONE) continue;
+        const int gg = (int)__float2uint_rz(__fmul_rn(g, 108.0f));
+        int rgb[3] = {(int)energy * 255 * p.smooth, gg * p.smooth, gg * p.smooth};
+#pragma unroll
+        for (int ch = 0; ch < 3; ++ch) {
+            const int old = col[3 * i + ch];
+            const int m = rgb[ch] < old + p.fade_in ? rgb[ch] : old + p.fade_in;
+            rgb[ch] = m > old - (int)(0u - (uint32_t)p.neg_fade_out) ? m : old - (int)(0u - (uint32_t)p.neg_fade_out);
+        }
+        col[3 * i] = rgb[0];
+        col[3 * i + 1] = rgb[1];
+        col[3 * i + 2] = rgb[2];
+        if (p.frame) {
+            // RendererPlain at zoom 1: the colour as a float, / SMOOTH_FACTOR,
+            // truncated, its low byte; exact without the division below 2^24
+            const bool small = (((uint32_t)rgb[0] + (1u << 24)) | ((uint32_t)rgb[1] + (1u << 24)) |
+                                ((uint32_t)rgb[2] + (1u << 24))) < (1u << 25);
+#pragma unroll
+            for (int ch = 0; ch < 3; ++ch) {
+                uint8_t px;
+                if (p.frame_smooth <= 1 && small) {
+                    px = (uint8_t)rgb[ch];
+                } else {
+                    float v = (float)rgb[ch];
+                    if (p.frame_smooth > 0) v = __fdiv_rn(v, (float)p.frame_smooth);
+                    px = (uint8_t)(int)v;
+                }
+                p.frame[3 * i + ch] = px;
+            }
+        }
     }
 }
 
@@ -415,12 +545,21 @@ cudaError_t xk_gravity_step(const uint64_t *src, uint64_t *dst, int32_t *col, co
     p.red = 255u * (uint32_t)d.smooth;
     p.frame = frame;
     p.frame_smooth = frame_smooth;
-    const dim3 block(XK_GC_THREADS);
+    // Four cells a thread where rows start on 16 bytes and the windows are two
+    // or more an SM: with fewer a generation takes 4.6 to 8.3 us by where the
+    // blocks land (640 x 360, 60 generations: 278 to 424 us, 333 x 222 500, against 412 and
+    // 400 one cell a thread), and colours by words gain nothing (1325 x 500
+    // 634 to 643 against 623 to 631).  1324 x 500 545 against 635, 1920 x 1080
+    // 1 010 against 1 300.
     p.tiles_x = (p.W + XK_GC_IX - 1) / XK_GC_IX;
-    const dim3 grid(p.tiles_x * ((p.H + XK_GC_IY - 1) / XK_GC_IY));
-    if (p.W % 4 == 0)       // rows of states and colours start on 16-byte boundaries, end on whole quads
-        return d.torus ? xk_launch_pdl(xk_k_gravity<true, true>, grid, block, 0, s, src, dst, col, p)
-                       : xk_launch_pdl(xk_k_gravity<false, true>, grid, block, 0, s, src, dst, col, p);
-    return d.torus ? xk_launch_pdl(xk_k_gravity<true, false>, grid, block, 0, s, src, dst, col, p)
-                   : xk_launch_pdl(xk_k_gravity<false, false>, grid, block, 0, s, src, dst, col, p);
+    const int64_t tiles = (int64_t)p.tiles_x * ((p.H + XK_GC_IY - 1) / XK_GC_IY);
+    if (p.W % 4 != 0 || tiles < 2 * (int64_t)xk_sm_count()) {
+        const dim3 one(XK_GC1_TX, XK_GC_THREADS / XK_GC1_TX);
+        const dim3 over((p.W + XK_GC1_TX - 1) / XK_GC1_TX, (p.H + XK_GC1_TY - 1) / XK_GC1_TY);
+        return d.torus ? xk_launch_pdl(xk_k_gravity_one<true>, over, one, 0, s, src, dst, col, p)
+                       : xk_launch_pdl(xk_k_gravity_one<false>, over, one, 0, s, src, dst, col, p);
+    }
+    const dim3 block(XK_GC_THREADS), grid((unsigned)tiles);
+    return d.torus ? xk_launch_pdl(xk_k_gravity<true>, grid, block, 0, s, src, dst, col, p)
+                   : xk_launch_pdl(xk_k_gravity<false>, grid, block, 0, s, src, dst, col, p);
 }
