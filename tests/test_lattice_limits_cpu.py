@@ -1,0 +1,49 @@
+"""Index arithmetic of the kernels at the widest lattices a model accepts
+(sides up to 2^31 - 1 cells).
+
+The functions that the kernels and their launchers share are compiled as host
+code with nvcc (no GPU needed) and checked against 64-bit arithmetic.
+"""
+import os
+import subprocess
+
+import pytest
+
+from tests.test_div_magic_cpu import CSRC, INCLUDE, _nvcc
+
+
+def _run(tmp_path, program):
+    nvcc = _nvcc()
+    if not nvcc:
+        pytest.skip("nvcc not found")
+    src, exe = str(tmp_path / "limits.cu"), str(tmp_path / "limits")
+    with open(src, "w") as fh:
+        fh.write(program)
+    subprocess.run([nvcc, "-std=c++17", "-O2", "-I", CSRC, "-I", INCLUDE, src, "-o", exe],
+                   check=True, capture_output=True, text=True)
+    return subprocess.run([exe], check=True, capture_output=True, text=True).stdout.split()
+
+
+def test_halves_of_a_rows_last_word(tmp_path):
+    """Rows of a multiple of 16 cells, up to 2^31 - 16: every word but an odd
+    row's last one has two halves."""
+    out = _run(tmp_path, r"""
+#include "xk_internal.cuh"
+#include <cstdio>
+
+int main()
+{
+    long long checked = 0, bad = 0;
+    for (int64_t W : {16ll, 32ll, 48ll, 1024ll, 1040ll, (1ll << 30) + 16, (1ll << 31) - 48, (1ll << 31) - 32,
+                      (1ll << 31) - 16}) {
+        const int64_t words = (W + 31) / 32;
+        for (int64_t j : {(int64_t)0, words / 2, words - 2, words - 1}) {
+            if (j < 0) continue;
+            ++checked;
+            bad += xk_word_halves((uint32_t)j, (int32_t)W) != (32 * j + 32 <= W ? 2 : 1);
+        }
+    }
+    std::printf("%lld %lld\n", checked, bad);
+}
+""")
+    assert int(out[0]) > 30 and int(out[1]) == 0

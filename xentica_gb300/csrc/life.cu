@@ -630,7 +630,7 @@ __global__ void xk_k_life_pack16(const uint8_t *__restrict__ src, uint32_t *__re
     if (word >= (uint32_t)g.H * (uint32_t)g.wpr) return;
     const uint32_t y = xk_divu(word, (uint32_t)g.wpr, g.div_wpr), j = word - y * (uint32_t)g.wpr;
     const uint4 *cells = (const uint4 *)(src + (int64_t)y * g.W + 32 * j);
-    const int halves = 32 * (int)j + 32 <= g.W ? 2 : 1;
+    const int halves = xk_word_halves(j, g.W);
     uint32_t bits = 0, over = 0;
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
@@ -654,7 +654,7 @@ __global__ void xk_k_life_unpack16(const uint32_t *__restrict__ src, uint8_t *__
     if (word >= (uint32_t)g.H * (uint32_t)g.wpr) return;
     const uint32_t y = xk_divu(word, (uint32_t)g.wpr, g.div_wpr), j = word - y * (uint32_t)g.wpr;
     uint4 *cells = (uint4 *)(dst + (int64_t)y * g.W + 32 * j);
-    const int halves = 32 * (int)j + 32 <= g.W ? 2 : 1;
+    const int halves = xk_word_halves(j, g.W);
     const uint32_t w = src[word];
     // four bits to four bytes: copies at 0, 7, 14, 21 put bit k at 8 k
     auto spread = [](uint32_t n) { return ((n & 0xFu) * 0x00204081u) & 0x01010101u; };

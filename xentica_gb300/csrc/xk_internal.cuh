@@ -89,6 +89,13 @@ __device__ __forceinline__ uint32_t xk_divu(uint32_t n, uint32_t d, uint32_t m)
     return m ? __umulhi(n, m) : n / d;
 }
 
+// 16-cell halves that word j of a row of W cells holds, W a multiple of 16
+// (unsigned: the words of the widest row end at 2^31)
+__host__ __device__ __forceinline__ int xk_word_halves(uint32_t j, int32_t W)
+{
+    return 32u * j + 32u <= (uint32_t)W ? 2 : 1;
+}
+
 LifeGeo xk_life_geo(int64_t W, int64_t H, int torus, int border_state);
 
 // one lattice (or ensemble instance) for the resident kernel
