@@ -47,3 +47,35 @@ int main()
 }
 """)
     assert int(out[0]) > 30 and int(out[1]) == 0
+
+
+@pytest.mark.parametrize("tile,halo", [(120, 4)])
+def test_columns_of_a_tile(tmp_path, tile, halo):
+    """Every column of the first and the last two tiles of a row, rows of one
+    cell to 2^31 - 1, as a kernel forms it modulo 2^32: inside the row or not,
+    and the wrapped one."""
+    out = _run(tmp_path, r"""
+#include "xk_internal.cuh"
+#include <cstdio>
+
+int main()
+{
+    const int64_t tile = %d, halo = %d;
+    long long checked = 0, bad = 0;
+    for (int64_t W : {1ll, 2ll, 3ll, 5ll, 119ll, 120ll, 121ll, 123ll, 240ll, 1000ll, (1ll << 31) - 250,
+                      (1ll << 31) - 129, (1ll << 31) - 128, (1ll << 31) - 64, (1ll << 31) - 9, (1ll << 31) - 1}) {
+        const int64_t tiles = (W + tile - 1) / tile;
+        for (int64_t t : {(int64_t)0, tiles - 2, tiles - 1})
+            for (int64_t off = -halo; off < tile + halo; ++off) {
+                if (t < 0) continue;
+                const int64_t x = t * tile + off, wrapped = ((x %% W) + W) %% W;
+                const uint32_t xu = (uint32_t)(t * tile) + (uint32_t)off;
+                const bool in = xu < (uint32_t)W;
+                ++checked;
+                bad += in != (x >= 0 && x < W) || (in ? (int)xu : xk_wrap_column(xu, (int)W)) != wrapped;
+            }
+    }
+    std::printf("%%lld %%lld\n", checked, bad);
+}
+""" % (tile, halo))
+    assert int(out[0]) > 4000 and int(out[1]) == 0

@@ -177,21 +177,20 @@ xk_k_lifecolor(const uint32_t *__restrict__ src, uint32_t *__restrict__ dst, int
     constexpr bool COLOR = COL != XK_LC_NONE;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int x0 = blockIdx.x * 120, y0 = blockIdx.y * p.TH, r0 = warp * R;
-    const int x = x0 - 4 + 4 * lane;                    // this lane's first cell
+    // this lane's first cell (compared unsigned: the tiles of the widest rows
+    // end beyond 2^31)
+    const uint32_t xu = (uint32_t)x0 + 4u * (uint32_t)lane - 4u;
+    const int x = (int)xu;
     int xs[4];
     bool xin[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        xs[k] = x + k;
-        xin[k] = xs[k] >= 0 && xs[k] < p.W;
-        if (TORUS && !xin[k]) {
-            xs[k] %= p.W;
-            if (xs[k] < 0) xs[k] += p.W;
-        }
+        xin[k] = xu + k < (uint32_t)p.W;
+        xs[k] = TORUS && !xin[k] ? xk_wrap_column(xu + k, p.W) : (int)(xu + k);
     }
     // the cells this thread keeps colours of and writes: inside the tile and
     // the lattice
-    const bool lin = lane >= 1 && lane <= 30 && x < p.W;
+    const bool lin = lane >= 1 && lane <= 30 && xu < (uint32_t)p.W;
     const bool quads = (p.W & 3) == 0;                  // rows start on 16 bytes
     // lanes 1 .. last store whole quads of pixels together
     const int last = min(30, (p.W - x0) >> 2);
@@ -415,10 +414,10 @@ cudaError_t xk_lifecolor_step(const uint32_t *src, uint32_t *dst, int32_t *col, 
     p.frame_smooth = frame_smooth;
     const int form = d.color_kind == XK_COLOR_NONE ? XK_LC_NONE
                      : lc_packs(d, color_range, frames, frame_smooth) ? XK_LC_PACKED : XK_LC_WIDE;
-    const int64_t gx = (p.W + 119) / 120;
+    const int64_t gx = ((int64_t)p.W + 119) / 120;
     auto tiles = [&](int R) {
         const int th = XK_LC_WARPS * R - 2 * p.T;
-        return gx * ((p.H + th - 1) / th);
+        return gx * (((int64_t)p.H + th - 1) / th);
     };
     // Rows a warp: of 5 and 4, the one whose waves of two blocks an SM cover
     // fewer rows; 2 where tiles of 4 would leave SMs without one (shorter

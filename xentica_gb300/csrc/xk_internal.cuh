@@ -96,6 +96,14 @@ __host__ __device__ __forceinline__ int xk_word_halves(uint32_t j, int32_t W)
     return 32u * j + 32u <= (uint32_t)W ? 2 : 1;
 }
 
+// Column of a torus row that x stands for, a column outside it: up to 2^29
+// beyond its end, or before its start (2^32 less the distance)
+__host__ __device__ __forceinline__ int xk_wrap_column(uint32_t x, int W)
+{
+    const int c = (int)(x < 0xC0000000u ? x - (uint32_t)W : x) % W;
+    return c < 0 ? c + W : c;
+}
+
 LifeGeo xk_life_geo(int64_t W, int64_t H, int torus, int border_state);
 
 // one lattice (or ensemble instance) for the resident kernel
