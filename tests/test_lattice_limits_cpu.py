@@ -79,3 +79,29 @@ int main()
 }
 """ % (tile, halo))
     assert int(out[0]) > 4000 and int(out[1]) == 0
+
+
+@pytest.mark.parametrize("side", [60, 64, 30, 16])
+def test_tiles_in_range(tmp_path, side):
+    """Where the rule for tiles holds, the farthest cell that the last tile
+    looks at (its start, its side, its halo, the cells loaded beside it: up to
+    64 on from its start, or 40 beyond it in rows) is an int; ordinary sides
+    are in range."""
+    out = _run(tmp_path, r"""
+#include "xk_internal.cuh"
+#include <cstdio>
+
+int main()
+{
+    const int64_t side = %d;
+    long long in = 0, bad = 0;
+    for (int64_t n = (1ll << 31) - 200; n < 1ll << 31; ++n) {
+        const int64_t start = (n - 1) / side * side;
+        if (!xk_tiles_in_range(n, 1) || !xk_tiles_in_range(1, n)) continue;
+        ++in;
+        bad += start + 64 > 0x7FFFFFFFll || n + side - 1 > 0x7FFFFFFFll;
+    }
+    std::printf("%%lld %%lld %%d\n", in, bad, (int)xk_tiles_in_range((1ll << 31) - 200, 1 << 30));
+}
+""" % side)
+    assert int(out[0]) > 100 and int(out[1]) == 0 and out[2] == "1"

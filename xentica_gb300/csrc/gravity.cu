@@ -551,9 +551,10 @@ cudaError_t xk_gravity_step(const uint64_t *src, uint64_t *dst, int32_t *col, co
     // 400 one cell a thread), and colours by words gain nothing (1325 x 500
     // 634 to 643 against 623 to 631).  1324 x 500 545 against 635, 1920 x 1080
     // 1 010 against 1 300.
-    p.tiles_x = (p.W + XK_GC_IX - 1) / XK_GC_IX;
-    const int64_t tiles = (int64_t)p.tiles_x * ((p.H + XK_GC_IY - 1) / XK_GC_IY);
-    if (p.W % 4 != 0 || tiles < 2 * (int64_t)xk_sm_count()) {
+    const int64_t tiles_x = ((int64_t)p.W + XK_GC_IX - 1) / XK_GC_IX;
+    const int64_t tiles = tiles_x * (((int64_t)p.H + XK_GC_IY - 1) / XK_GC_IY);
+    p.tiles_x = (int32_t)tiles_x;
+    if (p.W % 4 != 0 || !xk_tiles_in_range(p.W, p.H) || tiles < 2 * (int64_t)xk_sm_count()) {
         const dim3 one(XK_GC1_TX, XK_GC_THREADS / XK_GC1_TX);
         const dim3 over((p.W + XK_GC1_TX - 1) / XK_GC1_TX, (p.H + XK_GC1_TY - 1) / XK_GC1_TY);
         return d.torus ? xk_launch_pdl(xk_k_gravity_one<true>, over, one, 0, s, src, dst, col, p)

@@ -104,6 +104,13 @@ __host__ __device__ __forceinline__ int xk_wrap_column(uint32_t x, int W)
     return c < 0 ? c + W : c;
 }
 
+// Whether the coordinates of tiles of up to 64 cells a side, their halo and
+// the cells loaded beside it (64 in all beyond the last cell) are 32-bit ints
+__host__ __device__ constexpr bool xk_tiles_in_range(int64_t W, int64_t H)
+{
+    return W <= 0x7FFFFFFFll - 64 && H <= 0x7FFFFFFFll - 64;
+}
+
 LifeGeo xk_life_geo(int64_t W, int64_t H, int torus, int border_state);
 
 // one lattice (or ensemble instance) for the resident kernel
