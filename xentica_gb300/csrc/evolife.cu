@@ -752,7 +752,7 @@ cudaError_t xk_evolife_step(const uint64_t *src, uint64_t *dst, int32_t *col, co
     // them and 800 one a thread at 1280 x 720 (531 and 498 at 800 x 600, 257
     // and 190 at 320 x 200); with quads cut to words and bytes at 1919 x 1079
     // 1830 and 1626.
-    if (p.W % 4 != 0 || (int64_t)p.W * p.H < 3 << 18) {
+    if (p.W % 4 != 0 || !xk_tiles_in_range(p.W, p.H) || (int64_t)p.W * p.H < 3 << 18) {
         const dim3 block(32, 8), grid((p.W + 31) / 32, (p.H + 7) / 8);
         return p.mutation ? xk_launch_pdl(xk_k_evolife_one<true>, grid, block, 0, s, src, dst, col, p)
                           : xk_launch_pdl(xk_k_evolife_one<false>, grid, block, 0, s, src, dst, col, p);
