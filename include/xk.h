@@ -315,7 +315,11 @@ int xk_batch_step_noalloc(uint8_t *d_cells, int32_t count, const int32_t *width,
  * active request advances in rounds, a new round starting as soon as its
  * previous one finished, so requests admitted while others run share the GPU
  * with them.  Large 2-D, 3-D and mass-transfer lattices run rounds of
- * `quantum` generations on their own streams.  2-D lattices that fit one CTA
+ * `quantum` generations on their own streams; where `quantum` generations are
+ * short, a round takes several times as many, up to 4 (3-D Life-like lattices
+ * that a cluster holds up to 8), as long as it stays within about 3 ms of the
+ * request alone.  A cancelled request stops at the end of its round, and
+ * generations_done counts whole rounds.  2-D lattices that fit one CTA
  * run together, one resident-kernel launch per shape class over its idle
  * members (up to 4 such rounds of a class in flight), each member running
  * about quantum x 2^18 cell-generations per round (at least `quantum`

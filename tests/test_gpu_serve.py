@@ -186,3 +186,18 @@ def test_life3d_shapes(shape, generations):
     with serve.Server(1 << 28, quantum=16) as srv:
         got = srv.submit("life3d", cells, rule, generations).result(timeout=120)
     assert np.array_equal(got, oracle_result("life3d", cells, rule, generations))
+
+
+# quanta of 3 ms and more: 128 generations of 23 us (mass transfer), 2048 of 1.5
+# us (a large 2-D lattice, eight a launch), 2048 of more than 1.5 us on a cluster
+@pytest.mark.parametrize("kind,shape,rule,quantum,quanta", [
+    ("mass", (256, 280, 256), 0, 128, 4), ("life2d", (4096, 4096), 6152, 2048, 3),
+    ("life3d", (120, 128, 128), 0b0011000_0010100, 2048, 3)])
+def test_rounds_of_long_quanta_are_not_joined(kind, shape, rule, quantum, quanta):
+    """Where `quantum` generations already take milliseconds, a round is one
+    quantum: a cancelled request stops, and others get its SMs, that soon."""
+    cells = np.zeros(shape, dtype=np.uint32 if kind == "mass" else np.uint8)
+    cells.reshape(-1)[::7] = 1
+    with serve.Server(1 << 30, host_bytes=512 << 20, quantum=quantum) as srv:
+        srv.submit(kind, cells, rule, quanta * quantum).result(timeout=120)
+        assert srv.stats()["rounds"] >= quanta

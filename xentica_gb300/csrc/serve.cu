@@ -32,15 +32,16 @@
 //             members (one CTA each, each with its own generation count, about
 //             quantum x 2^18 cell-generations), in one of XK_SERVE_GROUP_SLOTS
 //             slots, so members admitted while a round runs start at once;
-//   global2d  larger 2-D lattices: packed to 32 cells per word once, one
-//             bit-sliced launch per generation on the request's stream;
+//   global2d  larger 2-D lattices: packed to 32 cells per word once, temporally
+//             blocked launches on the request's stream (XK_SERVE_TB generations
+//             each, 8 by default);
 //   life3d    3-D von Neumann Life-like: bit-packed along x like global2d, one
 //             launch per round on a cluster whose shared memory holds the
-//             lattice (8 x quantum generations a round), else one per
-//             generation;
+//             lattice, else one per generation;
 //   mass3d    mass transfer: uint32 ping-pong with the per-generation totals
 //             (the fast-only kernel when the submitted total is below 2^30).
-// The other paths run rounds of `quantum` generations.  Full rounds of the
+// The other paths run rounds of `quantum` generations, several of them in one
+// where they take a few milliseconds (round_quanta).  Full rounds of the
 // per-request paths are captured once as a CUDA graph (per ping-pong parity)
 // and replayed, so a round costs the worker one launch.  Streams carry a
 // priority: resident rounds the device's greatest, other requests one level
@@ -513,14 +514,41 @@ static int64_t round_flips(const Req *q, int64_t chunk)
     return chunk;
 }
 
+// Microseconds a generation of a request takes alone, to about a factor of
+// two, as its kernels measure: a cluster 1.4 up to 2048 words a CTA, 2.2 at
+// 4096; mass transfer below a total of 2^30 2.4 at 64^3, 10.6 at 7.5 M cells,
+// 21.2 at 16.8 M, above it about half as much again; eight generations a
+// launch of 4096 x 4096 1.5 each; other launches 1.6 at 65 536 words
+static double generation_us(const Req *q)
+{
+    if (q->path == PATH_MASS3D) return (q->mass_small ? 1.0 : 1.5) * (2.2 + 1.15e-6 * (double)q->n);
+    const double words = (double)q->lg.wpr * q->lg.H;
+    if (q->cl3.C) return 0.6 + words / q->cl3.C / 2560.0;
+    if (q->path == PATH_GLOBAL2D && q->tb_T > 1) return 0.4 + words / 480000.0;
+    return 1.2 + words / 160000.0;
+}
+
+// Quanta a request runs between two looks of the worker, at most `most`: as
+// many as take XK_SERVE_ROUND_US alone.  One after another they cost up to 40
+// us each until the worker has seen them end (13 % of 128 generations of a
+// small mass-transfer request, 1 % of 3 ms); a cancellation, and requests that
+// wait for the SMs, wait for the end of what was started.
+#define XK_SERVE_ROUND_US 3000.0
+static int64_t round_quanta(const xk_server *s, const Req *q, int64_t most)
+{
+    const double fit = XK_SERVE_ROUND_US / (generation_us(q) * (double)s->quantum);
+    return fit >= (double)most ? most : std::max<int64_t>(1, (int64_t)fit);
+}
+
 // next round of a request on its own stream; full rounds of requests with at
 // least two of them left are captured once per parity and replayed
 static int launch_round(xk_server *s, Req *q)
 {
-    const int64_t chunk = std::min(q->cl3.C ? 8 * s->quantum : s->quantum, q->r.generations - q->done);
+    const int64_t left = q->r.generations - q->done;
+    const int64_t chunk = std::min(q->cl3.C ? round_quanta(s, q, 8) * s->quantum : s->quantum, left);
     const int c0 = q->cur;
     const bool full = chunk == s->quantum && !q->cl3.C && graphs_enabled();
-    if (full && !q->graph[c0] && q->r.generations - q->done >= 2 * s->quantum) {
+    if (full && !q->graph[c0] && left >= 2 * s->quantum) {
         XK_CUDA(cudaStreamBeginCapture(q->stream, cudaStreamCaptureModeThreadLocal));
         int rc = enqueue_round(s, q, chunk);
         cudaGraph_t graph = nullptr;
@@ -538,11 +566,9 @@ static int launch_round(xk_server *s, Req *q)
     int64_t rounds = 1;
     if (full && q->graph[c0]) {
         // a graph that ends on the buffer it started from runs up to four
-        // times (about 2 ms of a small mass-transfer request, whose 128
-        // generations are followed by up to 40 us until this thread has seen
-        // them end)
+        // times
         if (round_flips(q, chunk) % 2 == 0)
-            rounds = std::min<int64_t>(4, (q->r.generations - q->done) / chunk);
+            rounds = std::min(round_quanta(s, q, 4), left / chunk);
         for (int64_t k = 0; k < rounds; ++k) XK_CUDA(cudaGraphLaunch(q->graph[c0], q->stream));
         q->cur = c0 ^ (int)(round_flips(q, chunk) & 1);
     } else {
