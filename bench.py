@@ -8,7 +8,10 @@ every lattice by 256 generations: one CUDA-graph launch of the resident
 kernel.  Inputs (~645 MB of cells, one byte each) exceed the 129 MB L2, so no
 flush is needed between steps.
 
-Reported (one JSON line on rank 0):
+Reported on rank 0, one JSON line of about 2000 characters, the last of the
+output (its ``value``, ``e2e``, ``roofline``, ``cpu_baseline``, ``clocks``,
+``parity`` and ``gpu_launches``); the rest before it, a line ``# name {...}``
+for each part:
   value   cell-updates/s over the K timed steps, device time (CUDA events on
           the launching stream), inputs resident in HBM;
   e2e     the same through ``xk_batch_run`` with pinned host buffers: every
@@ -393,6 +396,26 @@ def ensemble_parity(ens, widths, heights, G):
                     "against the oracle" % G}
 
 
+def headline(line):
+    """The short last line and the parts that are printed before it: a record
+    that keeps the end of the output has the whole line."""
+    short = dict(line)
+    parts = {k: short.pop(k) for k in ("plain", "reference_gpu", "seeding", "extras") if k in short}
+    parts.update(parts.pop("extras", {}))
+    for k in ("roofline", "parity", "cpu_baseline"):
+        if isinstance(short.get(k), dict):
+            parts[k] = short[k]
+            short[k] = {a: b for a, b in short[k].items() if a not in ("note", "bit_packed")}
+    return short, parts
+
+
+def report(line):
+    short, parts = headline(line)
+    for name, part in parts.items():
+        print("# %s %s" % (name, json.dumps(part)))
+    print(json.dumps(short), flush=True)
+
+
 def run_ours(args, dist):
     from xentica_gb300 import build as xk_build
     from xentica_gb300 import _native as nat
@@ -525,7 +548,7 @@ def run_ours(args, dist):
             if sub is not None:
                 line["extras"][name] = sub
     if dist.rank == 0:
-        print(json.dumps(line), flush=True)
+        report(line)
 
 
 def c2_experiment():
