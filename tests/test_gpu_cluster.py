@@ -170,3 +170,49 @@ def test_rows_exchanged_every_8_generations(cls, cluster, band):
             model.gpu.step(gens)
             O.life_run(topo, fld, np.zeros(3 * n, np.int32), gens)
             assert np.array_equal(model.gpu.arrays.cells.get()[:n], fld[:n]), (size, cluster, band, gens)
+
+
+# rules read from a table at run time (one with births in empty regions), a
+# border of dead cells and of live ones
+@pytest.mark.parametrize("band", [2, 3, 4, 6])
+@pytest.mark.parametrize("cluster", [2, 5, 16])
+@pytest.mark.parametrize("border", [None, 0, 1])
+@pytest.mark.parametrize("rule", ["B3/S23", "B36/S23", "B035/S1468"])
+def test_rows_exchanged_every_8_generations_any_rule(rule, border, cluster, band):
+    """The deep plan with a table's rule (and Conway's beside it), on a torus
+    and inside a border of either state: rows of several words, partial ones
+    among them, the last slab smaller."""
+    import ctypes
+    from xentica_gb300 import _native as nat
+    from xentica_gb300.tools.rules import LifeLike
+    from tests.models import GOLExperiment2, LifelikeFixed
+    code = LifeLike.golly2int(rule)
+    body = {}
+    if rule != "B3/S23":
+        body = {"rule": core.Parameter(default=code, interactive=True), "absorb": LifelikeFixed.absorb}
+    if border is not None:
+        body["Topology"] = type("Topology", (GameOfLife.Topology, ), {"border": core.StaticBorder(border)})
+    cls = type("Model", (GameOfLife, ), body)
+    ran = 0
+    for k, size in enumerate([(512, 512), (100, 301), (1000, 90), (31, 130)]):
+        model = cls(type("E", (GOLExperiment2, ), {"size": size, "zoom": 1, "rule": code}))
+        n = model.cells_num
+        cells = (np.random.RandomState(7 * cluster + k).random_sample(n) < 0.4).astype(np.uint8)
+        model.gpu.load(cells, np.zeros(3 * n, dtype=np.int32))
+        model.gpu._ensure()
+        model.gpu._planned = True
+        plan = (ctypes.c_int32 * 4)(4, cluster, band, 0)
+        if model.gpu._lib.xk_model_set_plan(model.gpu._handle, plan) != 0:
+            continue                            # no such cluster for this lattice
+        ran += 1
+        assert model.gpu._lib.xk_model_rule_form(model.gpu._handle) == (rule == "B3/S23")
+        topo = O.Topology(size, "moore", border)
+        fld = topo.field(cells, np.uint8)
+        for gens in (1, 8, 9, 41):
+            model.gpu.step(gens)
+            out = (ctypes.c_int32 * 4)()
+            nat.check(model.gpu._lib.xk_model_plan(model.gpu._handle, out), "xk_model_plan")
+            assert list(out) == [4, cluster, band, 0]
+            O.life_run(topo, fld, np.zeros(3 * n, np.int32), gens, born=code & 511, sustain=code >> 9)
+            assert np.array_equal(model.gpu.arrays.cells.get()[:n], fld[:n]), (size, gens)
+    assert ran
