@@ -76,3 +76,37 @@ def test_oracle_matches_the_interpreter_semantics():
             vm_cpu.step(model, b, cb, 6)
             assert np.array_equal(a[:n], b[:n]), (cls.__name__, size)
             assert np.array_equal(ca, cb), (cls.__name__, size)
+
+
+def test_mean_in_float_arithmetic():
+    """The kernel's quotient by 8.008 in float arithmetic (csrc/gravity.cu) for
+    every float of one binade, and near the ends of the range it is taken in:
+    the double division rounded to float, and none declined.  (Between those
+    ends a power of two scales every intermediate exactly.)  A fused
+    multiply-add is one in double here: each of its exact sums has at most 53
+    bits, checked by taking the sum's rounding error."""
+    ch, cl, r = (np.float32(float.fromhex(h)) for h in ("0x1.00418ap+3", "-0x1.916872p-22", "0x1.ff7d1p-4"))
+
+    def fma(a, b, c):
+        p, c = a.astype(np.float64) * np.float64(b), c.astype(np.float64)    # p: 48 bits, exact
+        s = p + c
+        back = s - p
+        assert not np.any((p - (s - back)) + (c - back))                     # what p + c lost
+        return s.astype(np.float32)
+
+    def check(f):
+        q1 = f * r
+        t = fma(-q1, cl, fma(-q1, ch, f)) * r
+        s = q1 + fma(q1, 2.0 ** -43, t)
+        assert np.array_equal(s, q1 + fma(q1, -2.0 ** -43, t))
+        assert np.array_equal(s, (f.astype(np.float64) / 8.008).astype(np.float32))
+
+    mantissas = np.arange(1 << 23, dtype=np.uint32)
+    for part in np.split(mantissas, 8):
+        f = (part | np.uint32(127 << 23)).view(np.float32)
+        check(f)
+    some = mantissas[::4099]
+    for e in (-60, -59, -1, 1, 60, 118, 119):
+        f = (some | np.uint32((127 + e) << 23)).view(np.float32)
+        check(f)
+        check(-f)
