@@ -202,6 +202,12 @@ int xk_vm_load(xk_model *m, int32_t which, const xk_vm_ins *code, int32_t ncode,
 /* Interactive parameter values (64-bit register images), bound at the next
  * step, as the reference passes them per launch (base.py:717, :722). */
 int xk_vm_set_params(xk_model *m, const uint64_t *values, int32_t count);
+/* The form program `which` runs in with the parameters bound now: */
+enum { XK_VM_FORM_NONE = 0,      /* none loaded, or not an interpreted model          */
+       XK_VM_FORM_WIDE = 1,      /* 64-bit values                                     */
+       XK_VM_FORM_NARROW = 2,    /* 32-bit values, the program a kernel argument      */
+       XK_VM_FORM_NARROW_LONG = 3 };   /* 32-bit values, too long for that            */
+int32_t xk_vm_form(const xk_model *m, int32_t which);
 
 /* Wait for all work queued on the model's stream. */
 int xk_sync(xk_model *m);

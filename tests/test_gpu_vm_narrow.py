@@ -216,3 +216,189 @@ def test_joined_operations(ty, swapped, again):
     col = np.zeros(3 * init.size, dtype=np.int32)
     want, got = _run(desc, (e, p), init, col, True), _run(desc, (e, p), init, col, False)
     assert np.array_equal(got[0], want[0])
+
+
+NONE, WIDE, NARROW, NARROW_LONG = range(4)
+
+
+class _Model:
+    """An interpreted model of two programs, narrow or (wide) held to the
+    64-bit form by one instruction of a 64-bit type in each."""
+
+    def __init__(self, desc, programs, init, col, wide=False):
+        self.lib, self.n, self.h = nat.load(), init.size, ctypes.c_void_p()
+        self.init, self.col = init, col
+        nat.check(self.lib.xk_model_create(ctypes.byref(desc), ctypes.byref(self.h)), "xk_model_create")
+        assert [self.form(w) for w in (0, 1)] == [NONE, NONE]
+        for which, p in enumerate(programs):
+            code = ([(O["const"], I64, p.nregs, 0, 0, 0, 0)] if wide else []) + list(p.code)
+            code = np.array(code, dtype=vm.INS_DTYPE)
+            consts = np.array(p.consts, dtype=np.uint64)
+            nat.check(self.lib.xk_vm_load(self.h, which, nat.ptr(code), len(code), nat.ptr(consts), len(consts),
+                                          p.nregs + 1), "xk_vm_load")
+        nat.check(self.lib.xk_upload(self.h, nat.ptr(init), self.n), "xk_upload")
+        nat.check(self.lib.xk_upload_colors(self.h, nat.ptr(col), self.n), "xk_upload_colors")
+        if wide:
+            assert [self.form(w) for w in (0, 1)] == [WIDE, WIDE]
+
+    def form(self, which):
+        return self.lib.xk_vm_form(self.h, which)
+
+    def bind(self, values):
+        v = np.array([x % 2 ** 64 for x in values], dtype=np.uint64)
+        nat.check(self.lib.xk_vm_set_params(self.h, nat.ptr(v), len(v)), "xk_vm_set_params")
+
+    def step(self, n):
+        nat.check(self.lib.xk_step(self.h, n), "xk_step")
+
+    def state(self):
+        cells, col = np.empty_like(self.init), np.empty_like(self.col)
+        nat.check(self.lib.xk_download(self.h, nat.ptr(cells), self.n), "xk_download")
+        nat.check(self.lib.xk_download_colors(self.h, nat.ptr(col), self.n), "xk_download_colors")
+        return cells, col
+
+    def frame(self, width, height):
+        img = np.empty(3 * width * height, dtype=np.int32)
+        nat.check(self.lib.xk_render(self.h, nat.ptr(img), width, height, 1, 0, 0), "xk_render")
+        return img.astype(np.uint8)
+
+    def __del__(self):
+        self.lib.xk_model_destroy(self.h)
+
+
+def _same(a, b):
+    for x, y in zip(a.state(), b.state()):
+        assert np.array_equal(x, y)
+
+
+def _program(code, consts=(0, ), ty=ir.U32, nregs=16):
+    return type("P", (), {"nregs": nregs, "code": code, "consts": [vm.pack_value(v, ty) for v in consts]})()
+
+
+def _desc(size, esz=4, **fields):
+    desc = nat.XkDesc()
+    desc.abi_version, desc.family, desc.ndim, desc.nbr = nat.XK_ABI_VERSION, nat.XK_FAMILY_VM, 2, 4
+    for d, s in enumerate(size):
+        desc.size[d] = s
+        desc.delta[2 * d][d], desc.delta[2 * d + 1][d] = 1, -1
+    desc.torus, desc.state_bytes, desc.proj_axis1 = 1, esz, 1
+    desc.color_kind, desc.fade_in, desc.fade_out, desc.smooth = nat.XK_COLOR_MOVING_AVERAGE, 40, 25, 2
+    for k, v in fields.items():
+        setattr(desc, k, v)
+    return desc
+
+
+# the main plane into every buffer
+COPY = _program([(O["load"], U32, 0, 0, 0, 0, 0)] + [(O["store"], U32, 0, 0, k, 0, 0) for k in range(1, 5)])
+
+
+# whole blocks of cells and a remainder, rows off 16 bytes, a frame of one row
+@pytest.mark.parametrize("size", [(64, 8), (67, 5), (257, 41), (333, 1)])
+@pytest.mark.parametrize("kind", [nat.XK_COLOR_MOVING_AVERAGE, nat.XK_COLOR_PLAIN])
+@pytest.mark.parametrize("render_smooth", [0, 1, 3])
+@pytest.mark.parametrize("scale", [1, 1 << 20])
+@pytest.mark.parametrize("where", ["host", "device"])
+def test_frames_of_the_absorb_pass(size, kind, render_smooth, scale, where):
+    """The zoom-1 frame of the whole lattice, written by the absorb pass:
+    colours that are their pixels, and ones beyond 2^24 and below 0, with and
+    without a division."""
+    desc = _desc(size, color_kind=kind, render_smooth=render_smooth)
+    absorb = _program(
+        [(O["load"], U32, k, 2, k, k + 1, 0) for k in range(4)] + [(O["load"], U32, 4, 0, 0, 0, 0)] +
+        [(O["const"], U32, 5, 0, 0, 0, 0), (O["const"], U32, 6, 1, 0, 0, 0), (O["const"], U32, 12, 2, 0, 0, 0)] +
+        [(O["+"], U32, 7, 0, 1, 0, 0), (O["+"], U32, 7, 7, 2, 0, 0), (O["+"], U32, 7, 7, 3, 0, 0)] +
+        [(O["^"], U32, 7, 7, 4, 0, 0), (O["&"], U32, 7, 7, 6, 0, 0), (O["store"], U32, 0, 7, 0, 0, 0)] +
+        [(O["*"], U32, 8, 7, 5, 0, 0), (O["*"], U32, 9, 4, 5, 0, 0), (O["-"], U32, 10, 12, 8, 0, 0)] +
+        [(O["color"], I32, 0, 8, 9, 10, 0)], (scale, 255, 90))
+    r = np.random.RandomState(size[0] + scale % 97)
+    n = size[0] * size[1]
+    init = r.randint(0, 256, n).astype(np.uint32)
+    col = r.randint(-100 * scale, 300 * scale, 3 * n).astype(np.int32)
+    a, b = _Model(desc, (COPY, absorb), init, col), _Model(desc, (COPY, absorb), init, col, wide=True)
+    assert [a.form(w) for w in (0, 1)] == [NARROW, NARROW]
+    steps = 6                       # more than the ring of host frames
+    want = np.empty((steps, 3 * n), dtype=np.uint8)
+    for g in range(steps):
+        b.step(1)
+        want[g] = b.frame(*size)
+    if where == "device":
+        torch = pytest.importorskip("torch")
+        out = torch.zeros(want.size, dtype=torch.uint8, device="cuda")
+        addr = out.data_ptr()
+    else:
+        out = np.zeros_like(want)
+        addr = out.ctypes.data
+    nat.check(a.lib.xk_step_frames(a.h, steps, size[0], size[1], 1, 0, 0, ctypes.c_void_p(addr),
+                                   int(where == "device")), "xk_step_frames")
+    got = out.cpu().numpy().reshape(want.shape) if where == "device" else out
+    assert np.array_equal(got, want)
+    _same(a, b)
+
+
+@pytest.mark.parametrize("nops,nconsts", [(128, 64), (129, 30), (100, 65), (1024, 64), (1025, 64), (3000, 300)])
+def test_program_lengths(nops, nconsts):
+    """Programs at the limits of each kernel argument, and beyond them."""
+    consts = [17 * k + 3 for k in range(nconsts - 1)]       # and the 0 of registers nobody wrote
+    code = [(O["load"], U32, 1, 0, 0, 0, 0)]
+    for k in range(nops - 2):
+        code.append((O["const"], U32, 2, k % len(consts), 0, 0, 0))
+        code.append((O["-" if k % 2 else "^"], U32, 1, 1, 2, 0, 0))
+    absorb = _program(code + [(O["store"], U32, 0, 1, 0, 0, 0)], consts)
+    desc = _desc((67, 5), color_kind=nat.XK_COLOR_NONE)
+    init = np.random.RandomState(nops).randint(0, 2 ** 32, 67 * 5, dtype=np.uint64).astype(np.uint32)
+    col = np.zeros(3 * init.size, dtype=np.int32)
+    a, b = _Model(desc, (COPY, absorb), init, col), _Model(desc, (COPY, absorb), init, col, wide=True)
+    assert [a.form(w) for w in (0, 1)] == [NARROW, NARROW if nops <= 1024 else NARROW_LONG]
+    for m in (a, b):
+        m.step(3)
+    _same(a, b)
+
+
+def test_parameters_rebound_in_and_out_of_32_bits():
+    """A bound parameter whose image is not the extension of its low half runs
+    the 64-bit form until one that is takes its place."""
+    absorb = _program(
+        [(O["load"], U32, 0, 0, 0, 0, 0), (O["param"], I32, 1, 0, 0, 0, 0), (O["param"], U32, 2, 3, 0, 0, 0)] +
+        [(O["const"], I32, 4, 0, 0, 0, 0), (O["<"], I32, 3, 1, 4, 0, 0)] +
+        [(O["+"], U32, 5, 0, 2, 0, 0), (O["cvt"], U32, 6, 1, I32, 0, 0)] +
+        [(O["/"], U32, 7, 5, 2, 0, 0), (O["^"], U32, 7, 7, 6, 0, 0), (O["+"], U32, 7, 7, 3, 0, 0)] +
+        [(O["store"], U32, 0, 7, 0, 0, 0), (O["color"], I32, 0, 3, 7, 1, 0)])
+    desc = _desc((33, 9))
+    r = np.random.RandomState(2)
+    init = r.randint(0, 2 ** 32, 33 * 9, dtype=np.uint64).astype(np.uint32)
+    col = r.randint(-500, 500, 3 * init.size).astype(np.int32)
+    a, b = _Model(desc, (COPY, absorb), init, col), _Model(desc, (COPY, absorb), init, col, wide=True)
+    for first, second, form in [(5, 7, NARROW), (-3, 2 ** 32 - 1, NARROW), (2 ** 40 + 1, 7, WIDE), (5, 7, NARROW),
+                                (5, 2 ** 32 + 9, WIDE), (2 ** 31, 1, WIDE), (-2 ** 31, 0, NARROW),
+                                (2 ** 31 - 1, 3, NARROW)]:
+        for m in (a, b):
+            m.bind((first, 0, 2 ** 63, second))
+            m.step(2)
+        assert [a.form(w) for w in (0, 1)] == [NARROW if form == NARROW else WIDE, form]
+        _same(a, b)
+
+
+@pytest.mark.parametrize("seed", range(24))
+def test_random_programs_that_translate(seed):
+    """Random programs that the 32-bit form takes (the first of a few draws
+    that it does): the form ran, and its cells and colours are the other's."""
+    desc = _desc([(64, 33), (5, 7), (1, 130)][seed % 3], [1, 2, 4][seed % 2 + seed % 3 // 2], torus=seed % 2,
+                 border_value=77)
+    n = desc.size[0] * desc.size[1]
+    r = np.random.RandomState(300 + seed)
+    init = r.randint(0, 200, n).astype({1: np.uint8, 2: np.uint16, 4: np.uint32}[desc.state_bytes])
+    col = r.randint(-500, 500, 3 * n).astype(np.int32)
+    for draw in range(30):
+        emit = _Random(100 * seed + draw, 4, desc.state_bytes, False)
+        emit.program(12, range(1, 5), False)
+        absorb = _Random(70000 + 100 * seed + draw, 4, desc.state_bytes, True)
+        absorb.program(50, [0], True)
+        a = _Model(desc, (emit, absorb), init, col)
+        if [a.form(w) for w in (0, 1)] == [NARROW, NARROW]:
+            break
+    else:
+        pytest.fail("no draw translated")
+    b = _Model(desc, (emit, absorb), init, col, wide=True)
+    for m in (a, b):
+        m.step(3)
+    _same(a, b)

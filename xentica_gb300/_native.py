@@ -119,6 +119,7 @@ SIGNATURES = {
     "xk_batch_step_noalloc": (_I32, [_P, _I32, _P, _P, _P, _I32, _P]),
     "xk_vm_load": (_I32, [_P, _I32, _P, _I32, _P, _I32, _I32]),
     "xk_vm_set_params": (_I32, [_P, _P, _I32]),
+    "xk_vm_form": (_I32, [_P, _I32]),
     "xk_serve_create": (_I32, [_I64, _I64, _I32, _I32, ctypes.POINTER(_P)]),
     "xk_serve_destroy": (_I32, [_P]),
     "xk_serve_request_bytes": (_I32, [ctypes.POINTER(XkRequest), ctypes.POINTER(_I64)]),

@@ -1608,3 +1608,10 @@ extern "C" int xk_vm_set_params(xk_model *m, const uint64_t *values, int32_t cou
     m->vm_params_fit = vm_params_fit(m);
     return XK_OK;
 }
+
+extern "C" int32_t xk_vm_form(const xk_model *m, int32_t which)
+{
+    if (!m || m->layout != LAYOUT_VM || which < 0 || which > 1 || m->vm_ncode[which] == 0) return XK_VM_FORM_NONE;
+    if (!m->vm_is_narrow[which] || !m->vm_params_fit) return XK_VM_FORM_WIDE;
+    return xk_vm_narrow_is_argument(m->vm_narrow[which]) ? XK_VM_FORM_NARROW : XK_VM_FORM_NARROW_LONG;
+}

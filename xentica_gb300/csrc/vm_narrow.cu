@@ -985,7 +985,7 @@ static cudaError_t vn_program(const VnParams &p, const XkVmNarrow &v, const uint
                               uint8_t *fld, int32_t *col, cudaStream_t s)
 {
     if (v.nops <= 128 && v.consts.size() <= 64) return vn_argument<ESZ, 128, 64>(p, v, fld, col, s);
-    if (v.nops <= 1024 && v.consts.size() <= 512) return vn_argument<ESZ, 1024, 512>(p, v, fld, col, s);
+    if (xk_vm_narrow_is_argument(v)) return vn_argument<ESZ, 1024, 512>(p, v, fld, col, s);
     const VnProgram<0, 0> prog = {(const XkVnCode *)code, consts};
     return vn_launch<ESZ>(p, prog, v, fld, col, s);
 }

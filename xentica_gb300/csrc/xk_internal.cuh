@@ -353,6 +353,8 @@ struct XkVmNarrow {
 };
 bool xk_vm_translate(const xk_vm_ins *code, int ncode, const uint64_t *consts, int nregs, const VmGeo &g,
                      XkVmNarrow *out);
+// whether it runs as a kernel argument (else from global memory)
+inline bool xk_vm_narrow_is_argument(const XkVmNarrow &v) { return v.nops <= 1024 && v.consts.size() <= 512; }
 cudaError_t xk_vm_run_narrow(const XkVmNarrow &v, const uint32_t *code, const uint32_t *consts,
                              const uint64_t *params, uint8_t *fld, int32_t *col, const VmGeo &g, cudaStream_t s,
                              uint8_t *frame = nullptr, int frame_smooth = 0);
