@@ -24,8 +24,10 @@
 // hold halo rows take them from the landing area, double-buffered by the same
 // parity.  A CTA sends exchange e + 2 only after it has received its
 // neighbours' e + 1, which they sent after reading their landing areas of e.
-// Waits are bounded (1 s): a CTA that gives up sets *gave_up and leaves the loop with all its threads; the last cluster
-// barrier keeps every CTA's shared memory alive until all are done.
+// Waits are bounded (1 s): a CTA that gives up sets *gave_up, leaves the loop
+// with all its threads and waits as long once more for rows that are still on
+// their way; the last cluster barrier keeps every CTA's shared memory alive
+// until all are done.
 //
 // Microseconds a generation, Conway's rule compiled in, 16 CTAs: 512 x 512 0.237
 // (cluster.cu 0.362, temporal blocking 0.389), 256 x 256 0.131 (0.329); 1000 x
@@ -160,8 +162,8 @@ xk_k_life_deep(uint32_t *__restrict__ bits, LifeGeo g, LifeTable9 t9, int genera
         }
     };
 
-    int left = generations;
-    for (int e = 0;; ++e) {
+    int left = generations, e = 0;
+    for (;; ++e) {
         const int n = min(left, K);
         for (int k = 0; k < n; k += 2) {
             generation(0);
@@ -198,6 +200,8 @@ xk_k_life_deep(uint32_t *__restrict__ bits, LifeGeo g, LifeTable9 t9, int genera
         // an even number of generations lies between exchanges, so the edge
         // rows' parities carry on
     }
+    // gave up: rows that are still on their way land while the CTA is there
+    if (left != 0) xk_cl_wait(mbar0 + 8u * ((uint32_t)e & 1u), (uint32_t)(e >> 1) & 1u);
     xk_cl_barrier_arrive();
     xk_cl_barrier_wait();
     if (!active) return;
