@@ -282,7 +282,7 @@ static bool deep_gave_up(xk_model *m)
 // Multi-generation steps of a 2-D lattice run in one launch on the resident
 // kernel (one CTA) or on a cluster of 2..16 CTAs (cluster.cu).  On the first
 // such step the candidates (cluster sizes, and bands of 1, 2 or 4 rows per
-// lane group) are timed over 32 generations on the ping-pong partner buffer
+// lane group) are timed over 48 generations on the ping-pong partner buffer
 // (the state is not touched), then clusters that exchange rows every 8
 // generations (cluster_deep.cu), and the fastest is kept; lattices too large for
 // one CTA take the fastest cluster that fits, else the per-generation global
@@ -784,10 +784,10 @@ extern "C" int xk_download(xk_model *m, void *host_main, int64_t ncells)
     return XK_OK;
 }
 
-// write the colours implied by the state into m->col
 // what a derived colour is its table's value times
 static int color_scale(const xk_model *m) { return m->d.color_kind == XK_COLOR_MOVING_AVERAGE ? m->d.smooth : 1; }
 
+// write the colours implied by the state into m->col
 static int materialize_colors(xk_model *m)
 {
     if (m->layout == LAYOUT_VM || m->layout == LAYOUT_LCOLOR || m->layout == LAYOUT_NOISE ||

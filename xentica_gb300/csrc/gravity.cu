@@ -34,7 +34,7 @@
 // colours beyond 2^24 moved out of line).
 //
 // 64 frames of 1920 x 1080: 1080 us, against 1410 of one cell a thread (its
-// 274 instructions a cell issued at 65 %; now 187, at 60 % of 42 % of the
+// 274 instructions a cell issued at 65 %; now 179, at 56 % of 43 % of the
 // warps: what is left to hide is the latency of one short launch a
 // generation).  Small lattices, and rows that do not start on 16
 // bytes, run one cell a thread (below).

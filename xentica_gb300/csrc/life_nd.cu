@@ -13,10 +13,13 @@
 // The six faces of a 3-D lattice have kernels of their own (life.cu,
 // life3d_cluster.cu): 100 generations of 128^3 450 -> 169 us.
 //
-// Bound by the launch, not by the arithmetic: a 128^3 lattice is 65 536 words
-// of about 210 instructions (0.35 us of issue on 152 SMs) and 262 KB that stay
-// in L2.  100 generations of 128^3 Moore and the read after them: 432 us,
-// against 18 468 us with the byte-per-cell kernel (xk_k_life_nd: one thread a
+// Bound by instruction issue: a word of 3-D Moore takes 1 073 instructions (its
+// 27 row words with their addresses and borders, the count, the rule's 63
+// selections), 1.9 us of issue on 152 SMs for the 65 536 words of 128^3, whose
+// 2 048 warps fill 58 % of the slots: 3.7 to 4 us a generation, where the
+// kernel of the six faces takes 1.6 in a launch of the same size.  100
+// generations of 128^3 Moore and the read after them: 425 us, against 18 468 us
+// with the byte-per-cell kernel (xk_k_life_nd: one thread a
 // cell, 27 loads with 64-bit coordinates), which is left for lattices this
 // packing cannot index.
 #include <string.h>

@@ -25,7 +25,7 @@
 // Bound by the logic pipe (63 %; 39 instructions a word, of which a rule read
 // from a table is 18) and by about 3 us a launch (its start, the tile's loads
 // and stores).  4096 x 4096, such a rule, 960 generations: 1 295 us with 12
-// generations a launch and tiles of 21 rows a warp (144 of the 152 SMs hold
+// generations a launch and tiles of 21 rows a warp (145 of the 152 SMs hold
 // one; 1 310 with 16 generations), 1 414 with 8, 1 605 with 8 on tiles of 12
 // rows a warp (two on most SMs, one on the others); twice that with the tile
 // in shared memory (every word of every generation loaded, stored and waited
