@@ -24,8 +24,8 @@
 // (tensor copies into a shared ring, a barrier a plane, 163 instructions a warp
 // and plane): 64^3 2.4 (3.4), 128^3 3.7 (5.5), 129 x 118 x 72 3.3 (5.5), 171 x
 // 205 x 215 10.6 (16.9), 256^3 21.2 (24.5; 25.2 with every generation marching
-// the same way); with a frame each 128^3 5.0 (7.5), 256^3 27.2 to 27.9 by the
-// box (29.9; 2 % more than now with the column sums in registers and the frame
+// the same way); with a frame each 128^3 5.0 (7.5), 256^3 27.2 to 27.9 from
+// run to run (29.9; 2 % more with the column sums in registers and the frame
 // before the first planes' loads).
 #include <string.h>
 
